@@ -13,6 +13,7 @@
 
 namespace cfk {
 cudaError_t launch_weno_air(const Zone &z, const Param &p, const int *var, cudaStream_t st, int *n_launch);
+int weno_air_default_tile(const Dims &d, int dir);
 cudaError_t launch_weno_air_dir(const Zone &z, const Param &p, int dir, int var, cudaStream_t st);
 cudaError_t weno_air_init_attributes();
 cudaError_t launch_pv_air(const Zone &z, const Param &p, cudaStream_t st, int *n_launch);
@@ -110,6 +111,15 @@ cudaError_t launch_inviscid(const Zone &z, const Param &p, const Thermo *th, con
     return th ? launch_weno_mix(z, p, *th, dt_dev, dt_host, var, st, n) : launch_weno_air(z, p, var, st, n);
   return th ? launch_pv_mix(z, p, *th, st, n) : launch_pv_air(z, p, st, n);
 }
+
+// Tile variants of the context's sweeps on its bound block.
+struct Tiles {
+  int var[3];
+  explicit Tiles(const cfk_ctx *c) {
+    for (int d = 0; d < 3; ++d)
+      var[d] = c->tile_auto && c->p.n_spec == 0 ? weno_air_default_tile(c->z.d, d) : c->tile_var[d];
+  }
+};
 
 // compute_viscous_flux dispatch (reference src/ViscousScheme.cu:7-73): the
 // 2nd-order face scheme or the 8th-order collocated one.
@@ -280,9 +290,8 @@ int cfk_create(const cfk_param *param, cfk_ctx **out) {
     p.limit_ul[l] = param->limit_ul[l];
   }
   // starting tile shapes and viscous form (cfk_autotune_tiles may change
-  // them): for air the ones the tuner picks on large 3-D blocks (x 31x8,
-  // y/z 31x16; the ring form with the L2 prefetch), for mixtures the first
-  // shape of each sweep
+  // them); until they are tuned or set, the air sweeps choose by the bound
+  // block's size instead (weno_air_default_tile)
   if (p.n_spec == 0) {
     c->tile_var[0] = 2;
     c->tile_var[1] = 1;
@@ -548,7 +557,7 @@ int cfk_compute_inviscid_flux(cfk_ctx *c, void *stream) {
   int n = 0;
   // the limiter's dt: the fixed dt, else the last CFL dt on the device
   const double *dt_dev = c->p.fixed_dt ? nullptr : reinterpret_cast<const double *>(c->d_dt_bits);
-  CFK_CHECK(c, launch_inviscid(c->z, c->p, thermo_host(c), dt_dev, c->hp.dt, c->tile_var, S(stream), &n),
+  CFK_CHECK(c, launch_inviscid(c->z, c->p, thermo_host(c), dt_dev, c->hp.dt, Tiles(c).var, S(stream), &n),
             "inviscid flux");
   c->launches += n;
   return CFK_OK;
@@ -637,6 +646,7 @@ int cfk_autotune_tiles(cfk_ctx *c, int reps, double *ms_out, int *choice_out, vo
   if (e != cudaSuccess) return cuda_fail(c, e, "autotune");
   c->visc_var = visc_choice;
   for (int d = 0; d < 3; ++d) c->tile_var[d] = choice[d];
+  c->tile_auto = false;
   if (choice_out) for (int d = 0; d < 3; ++d) choice_out[d] = choice[d];
   if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
   return CFK_OK;
@@ -660,6 +670,7 @@ int cfk_set_tile_variants(cfk_ctx *c, const int *var) {
   for (int d = 0; d < 3; ++d)
     if (var[d] < 0 || var[d] >= CFK_TILE_VARIANTS) return fail(c, CFK_ERR_ARG, "tile variant out of range");
   for (int d = 0; d < 3; ++d) c->tile_var[d] = var[d];
+  c->tile_auto = false;
   if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
   return CFK_OK;
 }
@@ -870,7 +881,7 @@ static int rk3_step_async(cfk_ctx *c, cudaStream_t st) {
     }
     {
       PhaseScope ps(c, CFK_PH_INVISCID, st, &n);
-      CFK_CHECK(c, launch_inviscid(z, p, thermo_host(c), dt_dev, c->hp.dt, c->tile_var, st, &n), "inviscid flux");
+      CFK_CHECK(c, launch_inviscid(z, p, thermo_host(c), dt_dev, c->hp.dt, Tiles(c).var, st, &n), "inviscid flux");
     }
     {
       PhaseScope ps(c, CFK_PH_UPDATE, st, &n);
@@ -970,7 +981,7 @@ static int wu_splitting(cfk_ctx *c, int schedule, const WuReaction &rx, double *
   }
   {
     PhaseScope ps(c, CFK_PH_INVISCID, st, &n);
-    CFK_CHECK(c, launch_inviscid(z, p, thermo_host(c), nullptr, dt, c->tile_var, st, &n), "inviscid flux");
+    CFK_CHECK(c, launch_inviscid(z, p, thermo_host(c), nullptr, dt, Tiles(c).var, st, &n), "inviscid flux");
     CFK_CHECK(c, cudaMemcpyAsync(z.Cn, z.dq, N * p.n_var * sizeof(double), cudaMemcpyDeviceToDevice, st),
               "Cn copy");
   }
@@ -1017,7 +1028,7 @@ static int wu_splitting(cfk_ctx *c, int schedule, const WuReaction &rx, double *
     }
     {
       PhaseScope ps(c, CFK_PH_INVISCID, st, &n);
-      CFK_CHECK(c, launch_inviscid(z, p, thermo_host(c), nullptr, dt, c->tile_var, st, &n), "inviscid flux");
+      CFK_CHECK(c, launch_inviscid(z, p, thermo_host(c), nullptr, dt, Tiles(c).var, st, &n), "inviscid flux");
     }
     {
       PhaseScope ps(c, CFK_PH_UPDATE, st, &n);

@@ -1,98 +1,119 @@
 // Scalar WENO5-JS / WENO7-Z reconstructions of the split characteristic
 // fluxes at i+1/2 (reference src/WENO.cu:3059-3222): same substencils,
-// smoothness indicators and weights; vp[] and vm[] run left to right and the
-// result is f+ + f-.  The weight normalisation is rearranged so that a face
-// costs one division per side pair instead of ten (WENO7) or six (WENO5).
+// smoothness indicators and weights, in exact arithmetic; vp[] and vm[] run
+// left to right and the result is f+ + f-.
 #pragma once
 
 namespace cfk {
 
-// WENO5-JS, f+ + f-.  The weights a_k = d_k / (eps + beta_k)^2 enter only
-// through sum(a_k v_k) / sum(a_k); both sums are multiplied through by the
-// product of the three denominators, so one division per side remains.  The
-// sides are not merged into one division: in flat regions the products are
-// O(eps^4) and their cross product would underflow.  Same reconstruction as
-// the reference; the rounding differs at the ulp level.
+// 1/x for x whose reciprocal is a normal number: the hardware's 20-bit
+// approximation (PTX rcp.approx.ftz.f64) and one third-order Householder step
+// y (1 + e + e^2), e = 1 - x y, whose remainder e^3 is below 2^-60; the result
+// is within 2 ulp.  Three FMAs, against a division sequence with its range
+// checks.  x = 0 and x = inf give NaN.
+__device__ __forceinline__ double rcp_nr(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// Dot products with a fixed order of FMAs.  Where the compiler chooses which
+// product of a sum to fuse, the choice can differ between the instantiations
+// of a kernel; the tile shapes of a sweep give bit-identical fluxes.
+__device__ __forceinline__ double dot2(double a0, double b0, double a1, double b1) { return fma(a0, b0, a1 * b1); }
+__device__ __forceinline__ double dot3(double a0, double b0, double a1, double b1, double a2, double b2) {
+  return fma(a0, b0, fma(a1, b1, a2 * b2));
+}
+// (the product with a zero addend rounds like the product alone)
+__device__ __forceinline__ double dot4p(double a0, double b0, double a1, double b1, double a2, double b2, double a3,
+                                        double b3, double plus) {
+  return fma(a0, b0, fma(a1, b1, fma(a2, b2, fma(a3, b3, plus))));
+}
+
+// WENO5-JS, f+ + f-.  Everything is formed from the differences of the stencil
+// values, d_i = u_{i+1} - u_i and s_i = d_{i+1} - d_i: the substencil values
+// are u2 plus a combination of them, the smoothness indicators
+// 13/12 s^2 + (first derivative)^2.  The weights a_k = d_k / (eps + beta_k)^2
+// enter only through sum(a_k v_k) / sum(a_k); both sums are multiplied through
+// by the product of the three denominators, so one division per side remains.
+// The sides are not merged into one division: in flat regions the products are
+// O(eps^4) and their cross product would underflow.
 __device__ __forceinline__ void weno5_side(double u0, double u1, double u2, double u3, double u4, double eps,
-                                           double d0, double d1, double d2, double &num, double &den) {
-  constexpr double one6th{1.0 / 6}, t12{13.0 / 12};
-  const double v0 = one6th * (2 * u2 + 5 * u3 - u4);
-  const double v1 = one6th * (-u1 + 5 * u2 + 2 * u3);
-  const double v2 = one6th * (2 * u0 - 7 * u1 + 11 * u2);
-  const double g0 = u2 + u4 - 2 * u3, h0 = 3 * u2 - 4 * u3 + u4;
-  const double g1 = u1 + u3 - 2 * u2, h1 = u1 - u3;
-  const double g2 = u0 + u2 - 2 * u1, h2 = u0 - 4 * u1 + 3 * u2;
-  const double b0 = eps + (t12 * g0 * g0 + 0.25 * h0 * h0);
-  const double b1 = eps + (t12 * g1 * g1 + 0.25 * h1 * h1);
-  const double b2 = eps + (t12 * g2 * g2 + 0.25 * h2 * h2);
-  const double D0 = b0 * b0, D1 = b1 * b1, D2 = b2 * b2;
-  const double a0 = d0 * (D1 * D2), a1 = d1 * (D0 * D2), a2 = d2 * (D0 * D1);
-  num = a0 * v0 + a1 * v1 + a2 * v2;
-  den = a0 + a1 + a2;
+                                           double &num, double &den) {
+  constexpr double one6th{1.0 / 6}, one3rd{1.0 / 3}, t12{13.0 / 12};
+  const double d0 = u1 - u0, d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3;
+  const double s0 = d1 - d0, s1 = d2 - d1, s2 = d3 - d2;
+  const double h0 = fma(-0.5, s2, d2), h1 = fma(0.5, s1, d1), h2 = fma(0.5, s0, d1);
+  const double b0 = fma(t12 * s2, s2, fma(h0, h0, eps));
+  const double b1 = fma(t12 * s1, s1, fma(h1, h1, eps));
+  const double b2 = fma(t12 * s0, s0, fma(h2, h2, eps));
+  const double m01 = b0 * b1, m02 = b0 * b2, m12 = b1 * b2;
+  const double a0 = (0.3 * m12) * m12, a1 = (0.6 * m02) * m02, a2 = (0.1 * m01) * m01;
+  const double hd = 0.5 * d2;
+  const double v0 = fma(-one6th, s2, hd), v1 = fma(-one6th, s1, hd), v2 = fma(one3rd, s0, 0.5 * d1);
+  num = fma(a2, v2, fma(a1, v1, a0 * v0));
+  den = __dadd_rn(__dadd_rn(a0, a1), a2);  // not contracted with the products
 }
 
 __device__ __forceinline__ double weno5_js(const double *vp, const double *vm, double eps) {
   double np, dp, nm, dm;
-  weno5_side(vp[0], vp[1], vp[2], vp[3], vp[4], eps, 0.3, 0.6, 0.1, np, dp);
+  weno5_side(vp[0], vp[1], vp[2], vp[3], vp[4], eps, np, dp);
   // mirrored: minus-side substencil k is plus-side substencil 2-k, same linear weights
-  weno5_side(vm[4], vm[3], vm[2], vm[1], vm[0], eps, 0.3, 0.6, 0.1, nm, dm);
-  return np / dp + nm / dm;
-}
-
-__device__ __forceinline__ double weno7_beta(double s1, double s2, double s3) {
-  constexpr double d12{13.0 / 12.0}, d13{1043.0 / 960}, d14{1.0 / 12};
-  return s1 * s1 + d12 * s2 * s2 + d13 * s3 * s3 + d14 * s1 * s3;
+  weno5_side(vm[4], vm[3], vm[2], vm[1], vm[0], eps, nm, dm);
+  return (vp[2] + vm[2]) + fma(np, rcp_nr(dp), nm * rcp_nr(dm));
 }
 
 // One side of WENO7-Z: u[0..6] ordered from the far upwind point to the far
-// downwind point of the stencil.  Returns numerator and denominator of
-// sum(a_k v_k) / sum(a_k) with a_k = c_k (1 + tau / (eps + beta_k)^2); the
-// four reciprocals are formed from two divisions, 1/(D0 D1) and 1/(D2 D3).
+// downwind point of the stencil, formed from the first, second and third
+// differences d, s, t of the values.  With s1', s2 and s3 the first (shifted by
+// s3 / 24), second and third differences at u3 of a substencil, the indicator
+// s1^2 + 13/12 s2^2 + 1043/960 s3^2 + s1 s3 / 12 is
+// s1'^2 + 13/12 s2^2 + 781/720 s3^2.  The weights c_k (1 + (T / e_k)^2),
+// e_k = eps + beta_k, T = e0 + 3 e1 - 3 e2 - e3, take one reciprocal, of
+// e0 e1 e2 e3 (>= eps^4, a normal number, see validate() in capi.cu; a product
+// of the squares would underflow in flat regions).  Returns numerator and
+// denominator of sum(a_k (v_k - u3)) / sum(a_k).  About 75 FP64 instructions
+// and one reciprocal a side, against 118 and two divisions when every
+// indicator and value is formed from the u[i].
 __device__ __forceinline__ void weno7_z_side(double u0, double u1, double u2, double u3, double u4, double u5,
                                              double u6, double eps, double &num, double &den) {
-  constexpr double one6th{1.0 / 6};
   constexpr double c0{1.0 / 35}, c1{12.0 / 35}, c2{18.0 / 35}, c3{4.0 / 35};
-  double s1 = one6th * (-2 * u0 + 9 * u1 - 18 * u2 + 11 * u3);
-  double s2 = -u0 + 4 * u1 - 5 * u2 + 2 * u3;
-  double s3 = -u0 + 3 * u1 - 3 * u2 + u3;
-  const double beta0 = weno7_beta(s1, s2, s3);
-  s1 = one6th * (u1 - 6 * u2 + 3 * u3 + 2 * u4);
-  s2 = u2 - 2 * u3 + u4;
-  s3 = -u1 + 3 * u2 - 3 * u3 + u4;
-  const double beta1 = weno7_beta(s1, s2, s3);
-  // stencil 2 shares the second difference of stencil 1 (reference src/WENO.cu:3137-3139)
-  s1 = one6th * (-2 * u2 - 3 * u3 + 6 * u4 - u5);
-  s3 = -u2 + 3 * u3 - 3 * u4 + u5;
-  const double beta2 = weno7_beta(s1, s2, s3);
-  s1 = one6th * (-11 * u3 + 18 * u4 - 9 * u5 + 2 * u6);
-  s2 = 2 * u3 - 5 * u4 + 4 * u5 - u6;
-  s3 = -u3 + 3 * u4 - 3 * u5 + u6;
-  const double beta3 = weno7_beta(s1, s2, s3);
-  double tau = beta0 + 3 * beta1 - 3 * beta2 - beta3;
-  tau *= tau;
-  const double e0 = eps + beta0, e1 = eps + beta1, e2 = eps + beta2, e3 = eps + beta3;
-  const double D0 = e0 * e0, D1 = e1 * e1, D2 = e2 * e2, D3 = e3 * e3;
-  const double r01 = 1.0 / (D0 * D1), r23 = 1.0 / (D2 * D3);
-  const double a0 = c0 + c0 * tau * (D1 * r01);
-  const double a1 = c1 + c1 * tau * (D0 * r01);
-  const double a2 = c2 + c2 * tau * (D3 * r23);
-  const double a3 = c3 + c3 * tau * (D2 * r23);
-  const double v0 = -3 * u0 + 13 * u1 - 23 * u2 + 25 * u3;
-  const double v1 = u1 - 5 * u2 + 13 * u3 + 3 * u4;
-  const double v2 = -u2 + 7 * u3 + 7 * u4 - u5;
-  const double v3 = 3 * u3 + 13 * u4 - 5 * u5 + u6;
-  num = a0 * v0 + a1 * v1 + a2 * v2 + a3 * v3;
-  den = a0 + a1 + a2 + a3;
+  constexpr double b2{13.0 / 12.0}, b3{781.0 / 720}, one3rd{1.0 / 3}, one6th{1.0 / 6}, one12th{1.0 / 12};
+  const double d0 = u1 - u0, d1 = u2 - u1, d2 = u3 - u2, d3 = u4 - u3, d4 = u5 - u4, d5 = u6 - u5;
+  const double s0 = d1 - d0, s1 = d2 - d1, s2 = d3 - d2, s3 = d4 - d3, s4 = d5 - d4;
+  const double t0 = s1 - s0, t1 = s2 - s1, t2 = s3 - s2, t3 = s4 - s3;
+  const double mid = fma(0.5, s2, d2);  // (u4 - u2) / 2
+  const double p0 = fma(0.375, t0, fma(0.5, s1, d2)), q0 = s1 + t0;
+  const double p1 = fma(-0.125, t1, mid), p2 = fma(-0.125, t2, mid);
+  const double p3 = fma(0.375, t3, fma(-0.5, s3, d3)), q3 = s3 - t3;
+  const double m12 = fma(b2 * s2, s2, eps);  // shared by the two middle substencils
+  const double e0 = fma(b3 * t0, t0, fma(b2 * q0, q0, fma(p0, p0, eps)));
+  const double e1 = fma(b3 * t1, t1, fma(p1, p1, m12));
+  const double e2 = fma(b3 * t2, t2, fma(p2, p2, m12));
+  const double e3 = fma(b3 * t3, t3, fma(b2 * q3, q3, fma(p3, p3, eps)));
+  const double tau = fma(3.0, e1 - e2, e0 - e3);
+  const double e01 = e0 * e1, e23 = e2 * e3;
+  const double r = rcp_nr(e01 * e23) * tau;
+  const double r01 = r * e23, r23 = r * e01;  // tau / (e0 e1), tau / (e2 e3)
+  const double w0 = r01 * e1, w1 = r01 * e0, w2 = r23 * e3, w3 = r23 * e2;
+  const double a0 = fma(c0 * w0, w0, c0), a1 = fma(c1 * w1, w1, c1);
+  const double a2 = fma(c2 * w2, w2, c2), a3 = fma(c3 * w3, w3, c3);
+  const double hd = 0.5 * d3, mv = fma(-one6th, s2, hd);
+  const double v0 = fma(0.25, t0, fma(one3rd, s1, 0.5 * d2));
+  const double v1 = fma(-one12th, t1, mv), v2 = fma(-one12th, t2, mv);
+  const double v3 = fma(one12th, t3, fma(-one6th, s3, hd));
+  num = fma(a3, v3, fma(a2, v2, fma(a1, v1, a0 * v0)));
+  den = (a0 + a1) + (a2 + a3);
 }
 
-// f+ + f-, one division shared by the two sides (each sum(a_k) >= 1/35, so
-// the product of the two denominators cannot underflow).
+// f+ + f-, one division shared by the two sides (each sum(a_k) >= 1, so the
+// product of the two denominators cannot underflow).
 __device__ __forceinline__ double weno7_z(const double *vp, const double *vm, double eps) {
   double np, dp, nm, dm;
   weno7_z_side(vp[0], vp[1], vp[2], vp[3], vp[4], vp[5], vp[6], eps, np, dp);
   weno7_z_side(vm[6], vm[5], vm[4], vm[3], vm[2], vm[1], vm[0], eps, nm, dm);
-  constexpr double one12th{1.0 / 12};
-  return one12th * ((np * dm + nm * dp) / (dp * dm));
+  return fma(fma(np, dm, nm * dp), rcp_nr(dp * dm), vp[3] + vm[3]);
 }
 
 // Linear branches of WENO5 / WENO7 used by the hybrid scheme away from

@@ -31,13 +31,18 @@ namespace {
 constexpr int kNQ = 13;  // staged values per point: Q0..4, G0..4, p, J/2, lambda
 
 // Tile shapes of a sweep: VAR selects one of the CFK_TILE_VARIANTS shapes
-// (nodes per column TN x columns C), chosen per direction by the tile
-// autotuner.  x tiles run along the lanes, y/z tiles put C consecutive i
-// columns on the lanes.
+// (nodes per column TN x columns C), chosen per direction by
+// weno_air_default_tile or the tile autotuner.  x tiles run along the lanes,
+// y/z tiles put C consecutive i columns on the lanes.  Tiles are small, one or
+// two faces a thread of a 128-thread CTA: four CTAs fit an SM and their
+// stage, face and difference phases overlap.  With the same 128 registers and
+// 16 warps an SM, two 256-thread CTAs took 984 us on the WENO7 sweeps of a
+// 161 x 113 x 97 block against 886; fewer warps with 168 registers took 990
+// (128 x 3) to 1100 (192 x 2).
 template <int DIR, int VAR>
 struct TileShape {
-  static constexpr int TN = DIR == 0 ? (VAR == 0 ? 63 : VAR == 1 ? 15 : 31) : (VAR == 0 ? 15 : VAR == 1 ? 31 : 63);
-  static constexpr int C = DIR == 0 ? (VAR == 0 ? 4 : VAR == 1 ? 16 : 8) : (VAR == 0 ? 32 : VAR == 1 ? 16 : 8);
+  static constexpr int TN = DIR == 0 ? (VAR == 0 ? 63 : VAR == 1 ? 15 : 31) : (VAR == 0 ? 31 : VAR == 1 ? 15 : 7);
+  static constexpr int C = DIR == 0 ? (VAR == 0 ? 2 : VAR == 1 ? 8 : 4) : (VAR == 0 ? 8 : VAR == 1 ? 16 : 16);
 };
 
 template <int DIR, int ORD, int VAR = 0>
@@ -48,7 +53,7 @@ struct AirTile {
   static constexpr int C = TileShape<DIR, VAR>::C;    // columns per CTA
   static constexpr int NF = TN + 1;             // faces per column
   static constexpr int NPT = TN + 2 * R + 2;    // staged points per column
-  static constexpr int NT = 256;                // threads
+  static constexpr int NT = 128;                // threads
   // shared-memory offset of (value q, column c, point/face t): x tiles are
   // column-major in t (lanes run along t), y/z tiles are row-major in c.
   __device__ static int spt(int q, int c, int t) {
@@ -63,26 +68,30 @@ struct AirTile {
 }  // namespace
 
 // The 13 staged values of one stencil point from its conserved variables,
-// p, T, the sweep's metric row and J.
+// p, T, the sweep's metric row and J: J/2 times Q and the Euler flux G (the
+// split fluxes need nothing else), p, 2/J (which gives the Roe average its
+// unscaled state back) and the spectral radius.
 template <class T>
 __device__ __forceinline__ void air_stage_point(double *s, int c, int t, double q0, double q1, double q2, double q3,
                                                 double q4, double pk, double tk, double m0, double m1, double m2,
                                                 double jac) {
-  const double Uk = (q1 * m0 + q2 * m1 + q3 * m2) / q0;
-  const double cGradK = norm3d(m0, m1, m2) * sqrt(kGammaAir * kRAir * tk);
+  const double Uk = dot3(q1, m0, q2, m1, q3, m2) * rcp_nr(q0);
+  const double lam = __dadd_rn(abs(Uk), sqrt(dot3(m0, m0, m1, m1, m2, m2) * (kGammaAir * kRAir * tk)));
+  const double hj = 0.5 * jac, hp = hj * pk;
+  q0 *= hj; q1 *= hj; q2 *= hj; q3 *= hj; q4 *= hj;
   s[T::spt(0, c, t)] = q0;
   s[T::spt(1, c, t)] = q1;
   s[T::spt(2, c, t)] = q2;
   s[T::spt(3, c, t)] = q3;
   s[T::spt(4, c, t)] = q4;
   s[T::spt(5, c, t)] = q0 * Uk;
-  s[T::spt(6, c, t)] = fma(q1, Uk, pk * m0);
-  s[T::spt(7, c, t)] = fma(q2, Uk, pk * m1);
-  s[T::spt(8, c, t)] = fma(q3, Uk, pk * m2);
-  s[T::spt(9, c, t)] = (q4 + pk) * Uk;
+  s[T::spt(6, c, t)] = fma(q1, Uk, hp * m0);
+  s[T::spt(7, c, t)] = fma(q2, Uk, hp * m1);
+  s[T::spt(8, c, t)] = fma(q3, Uk, hp * m2);
+  s[T::spt(9, c, t)] = __dadd_rn(q4, hp) * Uk;
   s[T::spt(10, c, t)] = pk;
-  s[T::spt(11, c, t)] = 0.5 * jac;
-  s[T::spt(12, c, t)] = abs(Uk) + cGradK;
+  s[T::spt(11, c, t)] = rcp_nr(hj);
+  s[T::spt(12, c, t)] = lam;
 }
 
 // Flux of the face between local points t + R and t + R + 1 of column c:
@@ -90,110 +99,125 @@ __device__ __forceinline__ void air_stage_point(double *s, int c, int t, double 
 // staged points, WENO (or, away from shocks in the hybrid scheme, the linear
 // upwind stencils) and back projection into sflx.  kx, ky, kz: the face
 // normal before normalisation.
+//
+// The five fields are taken as two pairs, the shear fields (1, 2) and the
+// acoustic ones (0, 4), and the entropy field 3: the two fields of a pair
+// share the loads of the staged points, which at one field at a time kept the
+// shared-memory pipe as busy as the FP64 one.  The pair loop is not unrolled:
+// unrolled, the stencil loads of all fields are hoisted above the first
+// field's arithmetic and spill; __syncwarp keeps them below it (so every lane
+// of a warp comes here, with valid = false where it has no face).  FP64-bound:
+// the three WENO7 sweeps of a 161 x 113 x 97 block went from 1217 to 793 us,
+// WENO5 of 200 x 150 x 150 from 2060 to 1270 us.
 template <int ORD, class T>
 __device__ __forceinline__ void air_face(const double *s, double *sflx, int c, int t, double kx, double ky, double kz,
-                                         double eps_ref, bool shock) {
+                                         double eps_ref, bool shock, bool valid) {
   constexpr int R = T::R, NPF = T::NPF;
   constexpr double gm1 = kGammaAir - 1;
+  auto recon = [&](const double *vp, const double *vm) -> double {
+    if constexpr (ORD == 7) return shock ? weno7_z(vp, vm, eps_ref) : weno7_linear(vp, vm);
+    else return shock ? weno5_js(vp, vm, eps_ref) : weno5_linear(vp, vm);
+  };
   const int pc = t + R;  // local point of node f
-    const double rho_l = s[T::spt(0, c, pc)], rho_r = s[T::spt(0, c, pc + 1)];
-    double temp1 = sqrt(rho_l * rho_r);
-    const double rlc = 1 / (rho_l + temp1);
-    const double rrc = 1 / (temp1 + rho_r);
-    const double um = rlc * s[T::spt(1, c, pc)] + rrc * s[T::spt(1, c, pc + 1)];
-    const double vm = rlc * s[T::spt(2, c, pc)] + rrc * s[T::spt(2, c, pc + 1)];
-    const double wm = rlc * s[T::spt(3, c, pc)] + rrc * s[T::spt(3, c, pc + 1)];
-    double temp3 = (rlc * s[T::spt(10, c, pc)] + rrc * s[T::spt(10, c, pc + 1)]) / kRAir;
-    const double cm = sqrt(kGammaAir * kRAir * temp3);
+  const double il = s[T::spt(11, c, pc)], ir = s[T::spt(11, c, pc + 1)];
+  const double rho_l = s[T::spt(0, c, pc)] * il, rho_r = s[T::spt(0, c, pc + 1)] * ir;
+  const double root = sqrt(rho_l * rho_r);
+  const double rlc = rcp_nr(__dadd_rn(rho_l, root)), rrc = rcp_nr(__dadd_rn(root, rho_r));
+  const double sl = rlc * il, sr = rrc * ir;  // weights of the scaled conserved variables
+  const double um = dot2(sl, s[T::spt(1, c, pc)], sr, s[T::spt(1, c, pc + 1)]);
+  const double vm = dot2(sl, s[T::spt(2, c, pc)], sr, s[T::spt(2, c, pc + 1)]);
+  const double wm = dot2(sl, s[T::spt(3, c, pc)], sr, s[T::spt(3, c, pc + 1)]);
+  const double pr = dot2(rlc, s[T::spt(10, c, pc)], rrc, s[T::spt(10, c, pc + 1)]);  // R T of the Roe average
+  const double H = fma(sl, s[T::spt(4, c, pc)], fma(sr, s[T::spt(4, c, pc + 1)], pr));
+  const double c2 = kGammaAir * pr, cm = sqrt(c2), ic2 = rcp_nr(c2);
 
-    temp1 = rnorm3d(kx, ky, kz);
-    kx *= temp1; ky *= temp1; kz *= temp1;
-    const double Uk_bar = kx * um + ky * vm + kz * wm;
-    double nx = 0, ny = 0, nz = 0;
-    if (abs(kx) > 0.8) { nx = -kz; nz = kx; }
-    else { ny = kz; nz = -ky; }
-    temp1 = rnorm3d(nx, ny, nz);
-    nx *= temp1; ny *= temp1; nz *= temp1;
-    double qx = ky * nz - kz * ny, qy = kz * nx - kx * nz, qz = kx * ny - ky * nx;
-    temp1 = rnorm3d(qx, qy, qz);
-    qx *= temp1; qy *= temp1; qz *= temp1;
-    const double Un = nx * um + ny * vm + nz * wm;
-    const double Uq = qx * um + qy * vm + qz * wm;
-    const double ic2 = 1.0 / (cm * cm);
-    const double alpha = 0.5 * gm1 * (um * um + vm * vm + wm * wm);
+  double nrm = rsqrt(dot3(kx, kx, ky, ky, kz, kz));
+  kx *= nrm; ky *= nrm; kz *= nrm;
+  const double Uk_bar = dot3(kx, um, ky, vm, kz, wm);
+  // rows of the two fields of a pair and their common energy coefficient,
+  // first the shear fields: n and q = k x n complete the basis
+  double A1 = 0, A2 = 0, A3 = 0;
+  if (abs(kx) > 0.8) { A1 = -kz; A3 = kx; }
+  else { A2 = kz; A3 = -ky; }
+  nrm = rsqrt(dot3(A1, A1, A2, A2, A3, A3));
+  A1 *= nrm; A2 *= nrm; A3 *= nrm;
+  double B1 = dot2(ky, A3, -kz, A2), B2 = dot2(kz, A1, -kx, A3), B3 = dot2(kx, A2, -ky, A1);
+  double A0 = -dot3(A1, um, A2, vm, A3, wm), B0 = -dot3(B1, um, B2, vm, B3, wm), E = 0;
+  const double alpha = 0.5 * gm1 * dot3(um, um, vm, vm, wm, wm);
 
-    double lam = 0;
+  double lam = 0;
 #pragma unroll
-    for (int q = 0; q < NPF; ++q) lam = max(lam, s[T::spt(12, c, t + q)]);
+  for (int q = 0; q < NPF; ++q) lam = max(lam, s[T::spt(12, c, t + q)]);
 
-    double fChar[5];
+  double f1 = 0, f2 = 0, f3 = 0, f4 = 0, ca, cb;
+#pragma unroll 1
+  for (int pair = 0;; ++pair) {
+    __syncwarp();
+    double va[NPF - 1], wa[NPF - 1], vb[NPF - 1], wb[NPF - 1];
 #pragma unroll
-    for (int l = 0; l < 5; ++l) {
-      // keep the stencil in shared memory across the five fields instead of
-      // letting the compiler hoist all 2R+2 points into registers
-      asm volatile("" ::: "memory");
-      double L0, L1, L2, L3, L4;
-      if (l == 0) {
-        L0 = (alpha + Uk_bar * cm) * ic2 * 0.5;
-        L1 = -(gm1 * um + kx * cm) * ic2 * 0.5;
-        L2 = -(gm1 * vm + ky * cm) * ic2 * 0.5;
-        L3 = -(gm1 * wm + kz * cm) * ic2 * 0.5;
-        L4 = gm1 * ic2 * 0.5;
-      } else if (l == 1) {
-        L0 = -Un; L1 = nx; L2 = ny; L3 = nz; L4 = 0;
-      } else if (l == 2) {
-        L0 = -Uq; L1 = qx; L2 = qy; L3 = qz; L4 = 0;
-      } else if (l == 3) {
-        L0 = 1 - alpha * ic2;
-        L1 = gm1 * um * ic2;
-        L2 = gm1 * vm * ic2;
-        L3 = gm1 * wm * ic2;
-        L4 = -gm1 * ic2;
-      } else {
-        L0 = (alpha - Uk_bar * cm) * ic2 * 0.5;
-        L1 = -(gm1 * um - kx * cm) * ic2 * 0.5;
-        L2 = -(gm1 * vm - ky * cm) * ic2 * 0.5;
-        L3 = -(gm1 * wm - kz * cm) * ic2 * 0.5;
-        L4 = gm1 * ic2 * 0.5;
-      }
-      double vp[NPF - 1], vmn[NPF - 1];
-#pragma unroll
-      for (int q = 0; q < NPF; ++q) {
-        const int tq = t + q;
-        double LF = L0 * s[T::spt(5, c, tq)] + L1 * s[T::spt(6, c, tq)] + L2 * s[T::spt(7, c, tq)] +
-                    L3 * s[T::spt(8, c, tq)];
-        double LQ = L0 * s[T::spt(0, c, tq)] + L1 * s[T::spt(1, c, tq)] + L2 * s[T::spt(2, c, tq)] +
-                    L3 * s[T::spt(3, c, tq)];
-        if (l != 1 && l != 2) {  // the rows of fields 1 and 2 have no energy term
-          LF += L4 * s[T::spt(9, c, tq)];
-          LQ += L4 * s[T::spt(4, c, tq)];
-        }
-        const double hj = s[T::spt(11, c, tq)];
-        if (q < NPF - 1) vp[q] = hj * (LF + lam * LQ);
-        if (q > 0) vmn[q - 1] = hj * (LF - lam * LQ);
-      }
-      if constexpr (ORD == 7) fChar[l] = shock ? weno7_z(vp, vmn, eps_ref) : weno7_linear(vp, vmn);
-      else fChar[l] = shock ? weno5_js(vp, vmn, eps_ref) : weno5_linear(vp, vmn);
+    for (int q = 0; q < NPF; ++q) {
+      const int tq = t + q;
+      const double g0 = s[T::spt(5, c, tq)], g1 = s[T::spt(6, c, tq)], g2 = s[T::spt(7, c, tq)],
+                   g3 = s[T::spt(8, c, tq)], eg = E * s[T::spt(9, c, tq)];
+      const double q0 = s[T::spt(0, c, tq)], q1 = s[T::spt(1, c, tq)], q2 = s[T::spt(2, c, tq)],
+                   q3 = s[T::spt(3, c, tq)], eq = E * s[T::spt(4, c, tq)];
+      const double Fa = dot4p(A0, g0, A1, g1, A2, g2, A3, g3, eg);
+      const double Fb = dot4p(B0, g0, B1, g1, B2, g2, B3, g3, eg);
+      const double Qa = dot4p(A0, q0, A1, q1, A2, q2, A3, q3, eq);
+      const double Qb = dot4p(B0, q0, B1, q1, B2, q2, B3, q3, eq);
+      if (q < NPF - 1) { va[q] = fma(lam, Qa, Fa); vb[q] = fma(lam, Qb, Fb); }
+      if (q > 0) { wa[q - 1] = fma(-lam, Qa, Fa); wb[q - 1] = fma(-lam, Qb, Fb); }
     }
-    // project back (right eigenvectors written out, reference src/WENO.cu:229-243)
-    const double f034 = fChar[0] + fChar[3] + fChar[4];
-    const double f04 = fChar[0] - fChar[4];
-    const double H = rlc * (s[T::spt(4, c, pc)] + s[T::spt(10, c, pc)]) +
-                     rrc * (s[T::spt(4, c, pc + 1)] + s[T::spt(10, c, pc + 1)]);
-    sflx[T::sfl(0, c, t)] = f034;
-    sflx[T::sfl(1, c, t)] = um * f034 - kx * cm * f04 + nx * fChar[1] + qx * fChar[2];
-    sflx[T::sfl(2, c, t)] = vm * f034 - ky * cm * f04 + ny * fChar[1] + qy * fChar[2];
-    sflx[T::sfl(3, c, t)] = wm * f034 - kz * cm * f04 + nz * fChar[1] + qz * fChar[2];
-    sflx[T::sfl(4, c, t)] = H * f034 - Uk_bar * cm * f04 + Un * fChar[1] + Uq * fChar[2] - cm * cm / gm1 * fChar[3];
+    ca = recon(va, wa);
+    cb = recon(vb, wb);
+    if (pair) break;
+    // back projection of the shear fields; next the acoustic pair
+    f1 = dot2(A1, ca, B1, cb);
+    f2 = dot2(A2, ca, B2, cb);
+    f3 = dot2(A3, ca, B3, cb);
+    f4 = -dot2(A0, ca, B0, cb);
+    const double h = 0.5 * ic2;
+    E = gm1 * h;
+    const double kc = cm * h, a0 = alpha * h;
+    A0 = fma(Uk_bar, kc, a0); A1 = -dot2(E, um, kx, kc); A2 = -dot2(E, vm, ky, kc); A3 = -dot2(E, wm, kz, kc);
+    B0 = fma(-Uk_bar, kc, a0); B1 = dot2(kx, kc, -E, um); B2 = dot2(ky, kc, -E, vm); B3 = dot2(kz, kc, -E, wm);
   }
+  const double f04 = cm * (ca - cb);
+  double f034 = ca + cb;
+  {
+    const double L4 = -gm1 * ic2, L0 = fma(-alpha, ic2, 1.0), L1 = -L4 * um, L2 = -L4 * vm, L3 = -L4 * wm;
+    __syncwarp();
+    double va[NPF - 1], wa[NPF - 1];
+#pragma unroll
+    for (int q = 0; q < NPF; ++q) {
+      const int tq = t + q;
+      const double F = dot4p(L0, s[T::spt(5, c, tq)], L1, s[T::spt(6, c, tq)], L2, s[T::spt(7, c, tq)], L3,
+                             s[T::spt(8, c, tq)], L4 * s[T::spt(9, c, tq)]);
+      const double Q = dot4p(L0, s[T::spt(0, c, tq)], L1, s[T::spt(1, c, tq)], L2, s[T::spt(2, c, tq)], L3,
+                             s[T::spt(3, c, tq)], L4 * s[T::spt(4, c, tq)]);
+      if (q < NPF - 1) va[q] = fma(lam, Q, F);
+      if (q > 0) wa[q - 1] = fma(-lam, Q, F);
+    }
+    const double c3 = recon(va, wa);
+    f034 += c3;
+    f4 = fma(-c2 * (1 / gm1), c3, f4);
+  }
+  if (!valid) return;
+  // right eigenvectors written out (reference src/WENO.cu:229-243)
+  sflx[T::sfl(0, c, t)] = f034;
+  sflx[T::sfl(1, c, t)] = fma(um, f034, fma(-kx, f04, f1));
+  sflx[T::sfl(2, c, t)] = fma(vm, f034, fma(-ky, f04, f2));
+  sflx[T::sfl(3, c, t)] = fma(wm, f034, fma(-kz, f04, f3));
+  sflx[T::sfl(4, c, t)] = fma(H, f034, fma(-Uk_bar, f04, f4));
+}
 
 // HYB: hybrid UD/WENO scheme, the face switches on the shock sensor.
 // VAR: tile shape (TileShape).
 template <int DIR, int ORD, bool HYB, int VAR>
-__global__ void __launch_bounds__(256, 2) weno_air_flux_diff(Zone z, double eps_ref, const double *sensor,
+__global__ void __launch_bounds__(128, 4) weno_air_flux_diff(Zone z, double eps_ref, const double *sensor,
                                                               double threshold) {
   using T = AirTile<DIR, ORD, VAR>;
-  constexpr int R = T::R, NPF = T::NPF, TN = T::TN, C = T::C, NF = T::NF, NPT = T::NPT;
+  constexpr int R = T::R, TN = T::TN, C = T::C, NF = T::NF, NPT = T::NPT;
   extern __shared__ double sm[];
   double *spts = sm;
   double *sflx = sm + kNQ * C * NPT;
@@ -243,16 +267,16 @@ __global__ void __launch_bounds__(256, 2) weno_air_flux_diff(Zone z, double eps_
     int c, t;
     split(item, NF, c, t);
     const int f = n0 - 1 + t;  // face between node f and f+1 along DIR
-    if (cbase + c >= ncol_max || f > m - 1) continue;
+    const bool valid = cbase + c < ncol_max && f < m;
     // face normal, averaged with the (i+1) node in every direction as the
     // reference does (reference src/WENO.cu:886-888, 1627-1629, 2303-2305)
-    const int64_t idf = node_idx(g, c, f);
+    const int64_t idf = valid ? node_idx(g, c, f) : 0;
     double kx = 0.5 * (z.metric[idf + mmo * sz] + z.metric[idf + 1 + mmo * sz]);
     double ky = 0.5 * (z.metric[idf + (mmo + 1) * sz] + z.metric[idf + 1 + (mmo + 1) * sz]);
     double kz = 0.5 * (z.metric[idf + (mmo + 2) * sz] + z.metric[idf + 1 + (mmo + 2) * sz]);
 
-    const bool shock = !HYB || face_shocked(sensor, idf, d.stride(g, DIR), g, threshold);
-    air_face<ORD, T>(spts, sflx, c, t, kx, ky, kz, eps_ref, shock);
+    const bool shock = !HYB || (valid && face_shocked(sensor, idf, d.stride(g, DIR), g, threshold));
+    air_face<ORD, T>(spts, sflx, c, t, kx, ky, kz, eps_ref, shock, valid);
   }
   __syncthreads();
 
@@ -264,7 +288,7 @@ __global__ void __launch_bounds__(256, 2) weno_air_flux_diff(Zone z, double eps_
     if (cbase + c >= ncol_max || a > m - 1) continue;
     const int64_t iq = node_idx(0, c, a);
 #pragma unroll
-    for (int v = 0; v < 5; ++v) z.dq[iq + v * szq] -= sflx[T::sfl(v, c, t + 1)] - sflx[T::sfl(v, c, t)];
+    for (int v = 0; v < 5; ++v) red_add(z.dq + iq + v * szq, sflx[T::sfl(v, c, t)] - sflx[T::sfl(v, c, t + 1)]);
   }
 }
 
@@ -332,6 +356,19 @@ cudaError_t launch_weno_air_dir(const Zone &z, const Param &p, int dir, int var,
   if (dir == 0) return w7 ? launch_dir<0, 7>(z, eps_ref, sn, th, var, st) : launch_dir<0, 5>(z, eps_ref, sn, th, var, st);
   if (dir == 1) return w7 ? launch_dir<1, 7>(z, eps_ref, sn, th, var, st) : launch_dir<1, 5>(z, eps_ref, sn, th, var, st);
   return w7 ? launch_dir<2, 7>(z, eps_ref, sn, th, var, st) : launch_dir<2, 5>(z, eps_ref, sn, th, var, st);
+}
+
+// The tile variant of a sweep that was neither tuned nor set.  On blocks of
+// more than one wave of CTAs (4 a SM) x 31x4, y 31x8 and z 15x16 are the
+// fastest (us per WENO7 sweep of 257 x 257 x 65, the three shapes: x 611, 586,
+// 565, y 592, 615, 621, z 741, 661, 670).  Below that a CTA's own latency
+// counts, and the y/z shape that takes its faces in one round instead of two
+// is faster (40 x 37 x 33: 18.6, 18.6, 14.5 us).
+int weno_air_default_tile(const Dims &d, int dir) {
+  if (dir == 0) return 2;
+  const long long ctas = (long long)((d.mx + 15) / 16) * ((d.ext(dir) + 14) / 15) * (dir == 1 ? d.mz : d.my);
+  if (ctas <= 4 * 148) return 2;
+  return dir == 1 ? 0 : 1;
 }
 
 // Host launcher: x, y and (3-D) z sweeps in the reference's order; var[d]

@@ -25,14 +25,19 @@ namespace cfk {
 
 namespace {
 
-// staged values per point: Q0..4, G0..4, U, p, J, lambda, rhoY[NS]
+// staged values per point: J/2 times Q0..4, the face-normal flux G0..4 and
+// rhoY[NS]; U, p, 2/J, lambda
 template <int NS>
 struct MixVals {
-  static constexpr int U = 10, P = 11, J = 12, LAM = 13, Y0 = 14, N = 14 + NS;
+  static constexpr int U = 10, P = 11, IJ = 12, LAM = 13, Y0 = 14, N = 14 + NS;
 };
 
 // Tile shapes of a sweep (nodes per column TN x columns C); VAR is chosen per
-// direction by the tile autotuner.
+// direction by the tile autotuner.  Every shape has 256 faces, one a thread,
+// and at 128 registers and 81 to 97 KB two CTAs fit an SM: FP64-bound.  With
+// all 14 fields unrolled a face took 226 registers, one CTA an SM, and its code
+// did not fit the instruction cache (WENO5 of 2048 x 512: 1786 -> 558 us;
+// WENO7 of 90 x 70 x 60: 1561 -> 485 us).
 template <int DIR, int VAR>
 struct MixShape {
   static constexpr int TN = DIR == 0 ? (VAR == 0 ? 63 : VAR == 1 ? 127 : 31) : (VAR == 0 ? 15 : VAR == 1 ? 31 : 63);
@@ -74,13 +79,14 @@ __device__ __noinline__ void pp_limit_x(const double *s, double *sf, int c, int 
   using T = MixTile<0, ORD, NS, VAR>;
   using V = MixVals<NS>;
   const int pc = t + T::R;
-  const double jac_l = s[T::spt(V::J, c, pc)], jac_r = s[T::spt(V::J, c, pc + 1)];
+  const double il = s[T::spt(V::IJ, c, pc)], ir = s[T::spt(V::IJ, c, pc + 1)];  // 2 / J: back to rho Y
+  const double jac_l = 2 / il, jac_r = 2 / ir;
   const double alphaL = 0.5 * alpha_dim * jac_l, alphaR = 0.5 * alpha_dim * jac_r;
   int start_l = -1;
   for (int l = 0; l < NS; ++l) {
     const double fl = sf[T::sfl(5 + l, c, t)];
-    const double up = alphaL * s[T::spt(V::Y0 + l, c, pc)] - dt * fl;
-    const double um = alphaR * s[T::spt(V::Y0 + l, c, pc + 1)] + dt * fl;
+    const double up = alphaL * (il * s[T::spt(V::Y0 + l, c, pc)]) - dt * fl;
+    const double um = alphaR * (ir * s[T::spt(V::Y0 + l, c, pc + 1)]) + dt * fl;
     if (up < 0 || um < 0) { start_l = l; break; }
   }
   if (start_l < 0) return;
@@ -98,7 +104,7 @@ __device__ __noinline__ void pp_limit_x(const double *s, double *sf, int c, int 
     const double fc = sf[T::sfl(5 + l, c, t)];
     double f1 = 0, theta_p = 1.0, theta_m = 1.0;
     bool f1_computed = false;
-    const double rhoYL = s[T::spt(V::Y0 + l, c, pc)], rhoYR = s[T::spt(V::Y0 + l, c, pc + 1)];
+    const double rhoYL = il * s[T::spt(V::Y0 + l, c, pc)], rhoYR = ir * s[T::spt(V::Y0 + l, c, pc + 1)];
     const double fp = 0.5 * jac_l * (UkL + cg[0]) * rhoYL;
     const double fm = 0.5 * jac_r * (UkR - cg[1]) * rhoYR;
     const double up = alphaL * rhoYL - dt * fc;
@@ -132,8 +138,9 @@ struct PPArgs {
 // HYB: hybrid UD/WENO scheme, the face switches on the shock sensor.
 // VAR: tile shape (MixShape).
 template <int DIR, int ORD, int NS, bool HYB, int VAR>
-__global__ void __launch_bounds__(256) weno_mix_flux_diff(Zone z, double eps_ref, const __grid_constant__ Thermo thermo,
-                                                          const double *sensor, double threshold, PPArgs pp) {
+__global__ void __launch_bounds__(256, 2) weno_mix_flux_diff(Zone z, double eps_ref,
+                                                             const __grid_constant__ Thermo thermo,
+                                                             const double *sensor, double threshold, PPArgs pp) {
   using T = MixTile<DIR, ORD, NS, VAR>;
   using V = MixVals<NS>;
   constexpr int R = T::R, NPF = T::NPF, TN = T::TN, C = T::C, NF = T::NF, NPT = T::NPT;
@@ -174,25 +181,26 @@ __global__ void __launch_bounds__(256) weno_mix_flux_diff(Zone z, double eps_ref
     const double q0 = z.cv[id], q1 = z.cv[id + sz], q2 = z.cv[id + 2 * sz], q3 = z.cv[id + 3 * sz],
                  q4 = z.cv[id + 4 * sz];
     const double m0 = z.metric[id + mmo * sz], m1 = z.metric[id + (mmo + 1) * sz], m2 = z.metric[id + (mmo + 2) * sz];
-    const double Uk = (q1 * m0 + q2 * m1 + q3 * m2) / q0;
-    const double pk = z.bv[id + 4 * sz];
+    const double Uk = dot3(q1, m0, q2, m1, q3, m2) * rcp_nr(q0);
+    const double pk = z.bv[id + 4 * sz], hj = 0.5 * z.jac[id], hp = hj * pk;
+    const double h0 = hj * q0, h1 = hj * q1, h2 = hj * q2, h3 = hj * q3, h4 = hj * q4;
     double *s = spts;
-    s[T::spt(0, c, t)] = q0;
-    s[T::spt(1, c, t)] = q1;
-    s[T::spt(2, c, t)] = q2;
-    s[T::spt(3, c, t)] = q3;
-    s[T::spt(4, c, t)] = q4;
-    s[T::spt(5, c, t)] = q0 * Uk;
-    s[T::spt(6, c, t)] = fma(q1, Uk, pk * m0);
-    s[T::spt(7, c, t)] = fma(q2, Uk, pk * m1);
-    s[T::spt(8, c, t)] = fma(q3, Uk, pk * m2);
-    s[T::spt(9, c, t)] = (q4 + pk) * Uk;
+    s[T::spt(0, c, t)] = h0;
+    s[T::spt(1, c, t)] = h1;
+    s[T::spt(2, c, t)] = h2;
+    s[T::spt(3, c, t)] = h3;
+    s[T::spt(4, c, t)] = h4;
+    s[T::spt(5, c, t)] = h0 * Uk;
+    s[T::spt(6, c, t)] = fma(h1, Uk, hp * m0);
+    s[T::spt(7, c, t)] = fma(h2, Uk, hp * m1);
+    s[T::spt(8, c, t)] = fma(h3, Uk, hp * m2);
+    s[T::spt(9, c, t)] = __dadd_rn(h4, hp) * Uk;
     s[T::spt(V::U, c, t)] = Uk;
     s[T::spt(V::P, c, t)] = pk;
-    s[T::spt(V::J, c, t)] = z.jac[id];
-    s[T::spt(V::LAM, c, t)] = abs(Uk) + sqrt(m0 * m0 + m1 * m1 + m2 * m2) * z.acoustic_speed[id];
+    s[T::spt(V::IJ, c, t)] = rcp_nr(hj);
+    s[T::spt(V::LAM, c, t)] = fma(sqrt(dot3(m0, m0, m1, m1, m2, m2)), z.acoustic_speed[id], abs(Uk));
 #pragma unroll
-    for (int l = 0; l < NS; ++l) s[T::spt(V::Y0 + l, c, t)] = z.cv[id + (5 + l) * sz];
+    for (int l = 0; l < NS; ++l) s[T::spt(V::Y0 + l, c, t)] = hj * z.cv[id + (5 + l) * sz];
   }
   __syncthreads();
 
@@ -201,160 +209,186 @@ __global__ void __launch_bounds__(256) weno_mix_flux_diff(Zone z, double eps_ref
     int c, t;
     split(item, NF, c, t);
     const int f = n0 - 1 + t;
-    if (cbase + c >= ncol_max || f > m - 1) continue;
+    const bool valid = cbase + c < ncol_max && f < m;
     const double *s = spts;
     const int pc = t + R;
+    auto recon = [&](const double *vp, const double *vm, bool shock) -> double {
+      if constexpr (ORD == 7) return shock ? weno7_z(vp, vm, eps_ref) : weno7_linear(vp, vm);
+      else return shock ? weno5_js(vp, vm, eps_ref) : weno5_linear(vp, vm);
+    };
     // face normal averaged with the (i+1) node, as the reference does
-    const int64_t idf = node_idx(g, c, f);
+    const int64_t idf = valid ? node_idx(g, c, f) : 0;
     double kx = 0.5 * (z.metric[idf + mmo * sz] + z.metric[idf + 1 + mmo * sz]);
     double ky = 0.5 * (z.metric[idf + (mmo + 1) * sz] + z.metric[idf + 1 + (mmo + 1) * sz]);
     double kz = 0.5 * (z.metric[idf + (mmo + 2) * sz] + z.metric[idf + 1 + (mmo + 2) * sz]);
+    const bool shock = !HYB || (valid && face_shocked(sensor, idf, d.stride(g, DIR), g, threshold));
 
-    const double rho_l = s[T::spt(0, c, pc)], rho_r = s[T::spt(0, c, pc + 1)];
-    double temp1 = sqrt(rho_l * rho_r);
-    const double rlc = 1 / (rho_l + temp1);
-    const double rrc = 1 / (temp1 + rho_r);
-    const double um = rlc * s[T::spt(1, c, pc)] + rrc * s[T::spt(1, c, pc + 1)];
-    const double vm = rlc * s[T::spt(2, c, pc)] + rrc * s[T::spt(2, c, pc + 1)];
-    const double wm = rlc * s[T::spt(3, c, pc)] + rrc * s[T::spt(3, c, pc + 1)];
-    double svm[NS];
+    const double il = s[T::spt(V::IJ, c, pc)], ir = s[T::spt(V::IJ, c, pc + 1)];
+    const double rho_l = s[T::spt(0, c, pc)] * il, rho_r = s[T::spt(0, c, pc + 1)] * ir;
+    const double root = sqrt(rho_l * rho_r);
+    const double rlc = rcp_nr(__dadd_rn(rho_l, root)), rrc = rcp_nr(__dadd_rn(root, rho_r));
+    const double sl = rlc * il, sr = rrc * ir;  // weights of the scaled conserved variables
+    const double um = dot2(sl, s[T::spt(1, c, pc)], sr, s[T::spt(1, c, pc + 1)]);
+    const double vm = dot2(sl, s[T::spt(2, c, pc)], sr, s[T::spt(2, c, pc + 1)]);
+    const double wm = dot2(sl, s[T::spt(3, c, pc)], sr, s[T::spt(3, c, pc + 1)]);
+    auto yk = [&](int l) { return dot2(sl, s[T::spt(V::Y0 + l, c, pc)], sr, s[T::spt(V::Y0 + l, c, pc + 1)]); };
+    const double pr = dot2(rlc, s[T::spt(V::P, c, pc)], rrc, s[T::spt(V::P, c, pc + 1)]);
+    const double H = fma(sl, s[T::spt(4, c, pc)], fma(sr, s[T::spt(4, c, pc + 1)], pr));
+    double rg = 0;
 #pragma unroll
-    for (int l = 0; l < NS; ++l)
-      svm[l] = rlc * s[T::spt(V::Y0 + l, c, pc)] + rrc * s[T::spt(V::Y0 + l, c, pc + 1)];
-    temp1 = 0;
-#pragma unroll
-    for (int l = 0; l < NS; ++l) temp1 += svm[l] * th->gas_const[l];
-    double temp3 = (rlc * s[T::spt(V::P, c, pc)] + rrc * s[T::spt(V::P, c, pc + 1)]) / temp1;
-    double hb[NS], cpb[NS];
-    enthalpy_cp_ns<NS>(th, temp3, hb, cpb);  // compute_enthalpy_and_cp at the averaged T
-    double temp2 = 0;
-#pragma unroll
-    for (int l = 0; l < NS; ++l) temp2 += svm[l] * cpb[l];
-    const double gamma = temp2 / (temp2 - temp1);
-    const double cm = sqrt(gamma * temp1 * temp3);
-    const double gm1 = gamma - 1;
-    temp1 = 1.0 / sqrt(kx * kx + ky * ky + kz * kz);
-    kx *= temp1; ky *= temp1; kz *= temp1;
-    const double Uk_bar = kx * um + ky * vm + kz * wm;
-    double nx = 0, ny = 0, nz = 0;
-    if (abs(kx) > 0.8) { nx = -kz; nz = kx; }
-    else { ny = kz; nz = -ky; }
-    temp1 = 1.0 / sqrt(nx * nx + ny * ny + nz * nz);
-    nx *= temp1; ny *= temp1; nz *= temp1;
-    double qx = ky * nz - kz * ny, qy = kz * nx - kx * nz, qz = kx * ny - ky * nx;
-    temp1 = 1.0 / sqrt(qx * qx + qy * qy + qz * qz);
-    qx *= temp1; qy *= temp1; qz *= temp1;
-    const double Un = nx * um + ny * vm + nz * wm;
-    const double Uq = qx * um + qy * vm + qz * wm;
-    temp2 = 1.0 / (cm * cm);
-    double beta[NS];
-#pragma unroll
+    for (int l = 0; l < NS; ++l) rg = fma(yk(l), th->gas_const[l], rg);
+    const double T3 = pr * rcp_nr(rg);
+    // h_l, then beta_l, wait in this face's species slots of the flux buffer;
+    // the loops over the species stay loops: unrolled, the face code of all
+    // fields overflows the instruction cache
+    double cps = 0;
+#pragma unroll 3
     for (int l = 0; l < NS; ++l) {
-      beta[l] = gamma * th->gas_const[l] * temp3 - gm1 * hb[l];
-      beta[l] *= temp2;
+      double h, cp;
+      enthalpy_cp_one(th, l, T3, h, cp);
+      cps = fma(yk(l), cp, cps);
+      sflx[T::sfl(5 + l, c, t)] = h;
     }
-    const double alpha = 0.5 * gm1 * (um * um + vm * vm + wm * wm);
+    const double gamma = cps / (cps - rg), gm1 = gamma - 1;
+    const double c2 = gamma * pr, cm = sqrt(c2), ic2 = rcp_nr(c2);
+#pragma unroll 3
+    for (int l = 0; l < NS; ++l)
+      sflx[T::sfl(5 + l, c, t)] = dot2(gamma * T3, th->gas_const[l], -gm1, sflx[T::sfl(5 + l, c, t)]) * ic2;
+
+    double nrm = rsqrt(dot3(kx, kx, ky, ky, kz, kz));
+    kx *= nrm; ky *= nrm; kz *= nrm;
+    const double Uk_bar = dot3(kx, um, ky, vm, kz, wm);
+    const double alpha = 0.5 * gm1 * dot3(um, um, vm, vm, wm, wm);
     double lam = 0;
 #pragma unroll
     for (int q = 0; q < NPF; ++q) lam = max(lam, s[T::spt(V::LAM, c, t + q)]);
-    const bool shock = !HYB || face_shocked(sensor, idf, d.stride(g, DIR), g, threshold);
-    double sbq[NPF], sbf[NPF];
-#pragma unroll
-    for (int q = 0; q < NPF; ++q) {
-      const int tq = t + q;
-      const double uq = s[T::spt(V::U, c, tq)];
-      double sp = 0, sn = 0;
-#pragma unroll
-      for (int n = 0; n < NS; ++n) {
-        const double ry = s[T::spt(V::Y0 + n, c, tq)];
-        sp = fma(beta[n], ry, sp);
-        sn = fma(beta[n], ry * uq, sn);
-      }
-      sbq[q] = sp;
-      sbf[q] = sn;
-    }
 
-    double fChar[5 + NS];
-#pragma unroll
-    for (int l = 0; l < 5; ++l) {
-      asm volatile("" ::: "memory");
-      double L0, L1, L2, L3, L4, tb = 0.5;
-      if (l == 0) {
-        L0 = (alpha + Uk_bar * cm) * temp2 * 0.5;
-        L1 = -(gm1 * um + kx * cm) * temp2 * 0.5;
-        L2 = -(gm1 * vm + ky * cm) * temp2 * 0.5;
-        L3 = -(gm1 * wm + kz * cm) * temp2 * 0.5;
-        L4 = gm1 * temp2 * 0.5;
-      } else if (l == 1) {
-        tb = 0; L0 = -Un; L1 = nx; L2 = ny; L3 = nz; L4 = 0;
-      } else if (l == 2) {
-        tb = 0; L0 = -Uq; L1 = qx; L2 = qy; L3 = qz; L4 = 0;
-      } else if (l == 3) {
-        tb = -1;
-        L0 = 1 - alpha * temp2;
-        L1 = gm1 * um * temp2;
-        L2 = gm1 * vm * temp2;
-        L3 = gm1 * wm * temp2;
-        L4 = -gm1 * temp2;
-      } else {
-        L0 = (alpha - Uk_bar * cm) * temp2 * 0.5;
-        L1 = -(gm1 * um - kx * cm) * temp2 * 0.5;
-        L2 = -(gm1 * vm - ky * cm) * temp2 * 0.5;
-        L3 = -(gm1 * wm - kz * cm) * temp2 * 0.5;
-        L4 = gm1 * temp2 * 0.5;
-      }
-      double vp[NPF - 1], vmn[NPF - 1];
+    // the fields in pairs that share the loads of the staged points, as in
+    // weno_air.cu; __syncwarp keeps the loads of a later block below the
+    // arithmetic of an earlier one
+    double f1, f2, f3, f4;
+    {  // shear fields: n and q = k x n complete the basis; no energy or species term
+      double A1 = 0, A2 = 0, A3 = 0;
+      if (abs(kx) > 0.8) { A1 = -kz; A3 = kx; }
+      else { A2 = kz; A3 = -ky; }
+      nrm = rsqrt(dot3(A1, A1, A2, A2, A3, A3));
+      A1 *= nrm; A2 *= nrm; A3 *= nrm;
+      const double B1 = dot2(ky, A3, -kz, A2), B2 = dot2(kz, A1, -kx, A3), B3 = dot2(kx, A2, -ky, A1);
+      const double A0 = -dot3(A1, um, A2, vm, A3, wm), B0 = -dot3(B1, um, B2, vm, B3, wm);
+      __syncwarp();
+      double va[NPF - 1], wa[NPF - 1], vb[NPF - 1], wb[NPF - 1];
 #pragma unroll
       for (int q = 0; q < NPF; ++q) {
         const int tq = t + q;
-        double LF = L0 * s[T::spt(5, c, tq)] + L1 * s[T::spt(6, c, tq)] + L2 * s[T::spt(7, c, tq)] +
-                    L3 * s[T::spt(8, c, tq)];
-        double LQ = L0 * s[T::spt(0, c, tq)] + L1 * s[T::spt(1, c, tq)] + L2 * s[T::spt(2, c, tq)] +
-                    L3 * s[T::spt(3, c, tq)];
-        if (l != 1 && l != 2) {  // the rows of fields 1 and 2 have no energy or species term
-          LF = LF + L4 * s[T::spt(9, c, tq)] + tb * sbf[q];
-          LQ = LQ + L4 * s[T::spt(4, c, tq)] + tb * sbq[q];
-        }
-        const double jq = s[T::spt(V::J, c, tq)];
-        if (q < NPF - 1) vp[q] = 0.5 * jq * (LF + lam * LQ);
-        if (q > 0) vmn[q - 1] = 0.5 * jq * (LF - lam * LQ);
+        const double g0 = s[T::spt(5, c, tq)], g1 = s[T::spt(6, c, tq)], g2 = s[T::spt(7, c, tq)],
+                     g3 = s[T::spt(8, c, tq)];
+        const double q0 = s[T::spt(0, c, tq)], q1 = s[T::spt(1, c, tq)], q2 = s[T::spt(2, c, tq)],
+                     q3 = s[T::spt(3, c, tq)];
+        const double Fa = dot4p(A1, g1, A2, g2, A3, g3, A0, g0, 0.0), Fb = dot4p(B1, g1, B2, g2, B3, g3, B0, g0, 0.0);
+        const double Qa = dot4p(A1, q1, A2, q2, A3, q3, A0, q0, 0.0), Qb = dot4p(B1, q1, B2, q2, B3, q3, B0, q0, 0.0);
+        if (q < NPF - 1) { va[q] = fma(lam, Qa, Fa); vb[q] = fma(lam, Qb, Fb); }
+        if (q > 0) { wa[q - 1] = fma(-lam, Qa, Fa); wb[q - 1] = fma(-lam, Qb, Fb); }
       }
-      if constexpr (ORD == 7) fChar[l] = shock ? weno7_z(vp, vmn, eps_ref) : weno7_linear(vp, vmn);
-      else fChar[l] = shock ? weno5_js(vp, vmn, eps_ref) : weno5_linear(vp, vmn);
+      const double ca = recon(va, wa, shock), cb = recon(vb, wb, shock);
+      f1 = dot2(A1, ca, B1, cb);
+      f2 = dot2(A2, ca, B2, cb);
+      f3 = dot2(A3, ca, B3, cb);
+      f4 = -dot2(A0, ca, B0, cb);
     }
+    __syncwarp();
+    double sb[NPF];  // sum of beta_k rho Y_k at the stencil points; their flux is U times it
+    {
+      double beta[NS];
 #pragma unroll
-    for (int l = 0; l < NS; ++l) {
-      asm volatile("" ::: "memory");
-      double vp[NPF - 1], vmn[NPF - 1];
+      for (int l = 0; l < NS; ++l) beta[l] = sflx[T::sfl(5 + l, c, t)];
+#pragma unroll
+      for (int q = 0; q < NPF; ++q) {
+        sb[q] = 0;
+#pragma unroll
+        for (int l = 0; l < NS; ++l) sb[q] = fma(beta[l], s[T::spt(V::Y0 + l, c, t + q)], sb[q]);
+      }
+    }
+    double f04, f034;
+    {  // acoustic fields
+      const double h = 0.5 * ic2, E = gm1 * h, kc = cm * h, a0 = alpha * h;
+      const double A0 = fma(Uk_bar, kc, a0), B0 = fma(-Uk_bar, kc, a0);
+      const double A1 = -dot2(E, um, kx, kc), A2 = -dot2(E, vm, ky, kc), A3 = -dot2(E, wm, kz, kc);
+      const double B1 = dot2(kx, kc, -E, um), B2 = dot2(ky, kc, -E, vm), B3 = dot2(kz, kc, -E, wm);
+      __syncwarp();
+      double va[NPF - 1], wa[NPF - 1], vb[NPF - 1], wb[NPF - 1];
 #pragma unroll
       for (int q = 0; q < NPF; ++q) {
         const int tq = t + q;
-        const double LQ = s[T::spt(V::Y0 + l, c, tq)] - svm[l] * s[T::spt(0, c, tq)];
-        const double LF = s[T::spt(V::U, c, tq)] * LQ;
-        const double jq = s[T::spt(V::J, c, tq)];
-        if (q < NPF - 1) vp[q] = 0.5 * jq * (LF + lam * LQ);
-        if (q > 0) vmn[q - 1] = 0.5 * jq * (LF - lam * LQ);
+        const double hs = 0.5 * sb[q];
+        const double g0 = s[T::spt(5, c, tq)], g1 = s[T::spt(6, c, tq)], g2 = s[T::spt(7, c, tq)],
+                     g3 = s[T::spt(8, c, tq)], eg = fma(E, s[T::spt(9, c, tq)], s[T::spt(V::U, c, tq)] * hs);
+        const double q0 = s[T::spt(0, c, tq)], q1 = s[T::spt(1, c, tq)], q2 = s[T::spt(2, c, tq)],
+                     q3 = s[T::spt(3, c, tq)], eq = fma(E, s[T::spt(4, c, tq)], hs);
+        const double Fa = dot4p(A0, g0, A1, g1, A2, g2, A3, g3, eg);
+        const double Fb = dot4p(B0, g0, B1, g1, B2, g2, B3, g3, eg);
+        const double Qa = dot4p(A0, q0, A1, q1, A2, q2, A3, q3, eq);
+        const double Qb = dot4p(B0, q0, B1, q1, B2, q2, B3, q3, eq);
+        if (q < NPF - 1) { va[q] = fma(lam, Qa, Fa); vb[q] = fma(lam, Qb, Fb); }
+        if (q > 0) { wa[q - 1] = fma(-lam, Qa, Fa); wb[q - 1] = fma(-lam, Qb, Fb); }
       }
-      if constexpr (ORD == 7) fChar[5 + l] = shock ? weno7_z(vp, vmn, eps_ref) : weno7_linear(vp, vmn);
-      else fChar[5 + l] = shock ? weno5_js(vp, vmn, eps_ref) : weno5_linear(vp, vmn);
+      const double ca = recon(va, wa, shock), cb = recon(vb, wb, shock);
+      f04 = cm * (ca - cb);
+      f034 = ca + cb;
     }
-    const double f034 = fChar[0] + fChar[3] + fChar[4];
-    const double f04 = fChar[0] - fChar[4];
-    const double H = rlc * (s[T::spt(4, c, pc)] + s[T::spt(V::P, c, pc)]) +
-                     rrc * (s[T::spt(4, c, pc + 1)] + s[T::spt(V::P, c, pc + 1)]);
-    sflx[T::sfl(0, c, t)] = f034;
-    sflx[T::sfl(1, c, t)] = um * f034 - kx * cm * f04 + nx * fChar[1] + qx * fChar[2];
-    sflx[T::sfl(2, c, t)] = vm * f034 - ky * cm * f04 + ny * fChar[1] + qy * fChar[2];
-    sflx[T::sfl(3, c, t)] = wm * f034 - kz * cm * f04 + nz * fChar[1] + qz * fChar[2];
-    double f4 = H * f034 - Uk_bar * cm * f04 + Un * fChar[1] + Uq * fChar[2] - cm * cm / gm1 * fChar[3];
+    {  // entropy field
+      const double L4 = -gm1 * ic2, L0 = fma(-alpha, ic2, 1.0), L1 = -L4 * um, L2 = -L4 * vm, L3 = -L4 * wm;
+      __syncwarp();
+      double va[NPF - 1], wa[NPF - 1];
+#pragma unroll
+      for (int q = 0; q < NPF; ++q) {
+        const int tq = t + q;
+        const double F = dot4p(L0, s[T::spt(5, c, tq)], L1, s[T::spt(6, c, tq)], L2, s[T::spt(7, c, tq)], L3,
+                               s[T::spt(8, c, tq)], dot2(L4, s[T::spt(9, c, tq)], -s[T::spt(V::U, c, tq)], sb[q]));
+        const double Q = dot4p(L0, s[T::spt(0, c, tq)], L1, s[T::spt(1, c, tq)], L2, s[T::spt(2, c, tq)], L3,
+                               s[T::spt(3, c, tq)], fma(L4, s[T::spt(4, c, tq)], -sb[q]));
+        if (q < NPF - 1) va[q] = fma(lam, Q, F);
+        if (q > 0) wa[q - 1] = fma(-lam, Q, F);
+      }
+      const double c3 = recon(va, wa, shock);
+      f034 += c3;
+      f4 = fma(-c2 / gm1, c3, f4);
+    }
+    if (valid) {
+      sflx[T::sfl(0, c, t)] = f034;
+      sflx[T::sfl(1, c, t)] = fma(um, f034, fma(-kx, f04, f1));
+      sflx[T::sfl(2, c, t)] = fma(vm, f034, fma(-ky, f04, f2));
+      sflx[T::sfl(3, c, t)] = fma(wm, f034, fma(-kz, f04, f3));
+    }
+    f4 = fma(H, f034, fma(-Uk_bar, f04, f4));
+    // species fields rho Y_k - Y~_k rho: their fluxes are U times them
+    __syncwarp();
     double bsum = 0;
+    {
+      double q0[NPF], up[NPF], dn[NPF];
 #pragma unroll
-    for (int l = 0; l < NS; ++l) {
-      sflx[T::sfl(5 + l, c, t)] = svm[l] * f034 + fChar[5 + l];
-      bsum += beta[l] * fChar[5 + l];
+      for (int q = 0; q < NPF; ++q) {
+        const double U = s[T::spt(V::U, c, t + q)];
+        q0[q] = s[T::spt(0, c, t + q)];
+        up[q] = U + lam;
+        dn[q] = U - lam;
+      }
+#pragma unroll 1
+      for (int l = 0; l < NS; ++l) {
+        const double y = yk(l);
+        double va[NPF - 1], wa[NPF - 1];
+#pragma unroll
+        for (int q = 0; q < NPF; ++q) {
+          const double w = fma(-y, q0[q], s[T::spt(V::Y0 + l, c, t + q)]);
+          if (q < NPF - 1) va[q] = up[q] * w;
+          if (q > 0) wa[q - 1] = dn[q] * w;
+        }
+        const double cs = recon(va, wa, shock);
+        bsum = fma(sflx[T::sfl(5 + l, c, t)], cs, bsum);
+        sflx[T::sfl(5 + l, c, t)] = fma(y, f034, cs);
+      }
     }
-    f4 -= bsum * cm * cm / gm1;
-    sflx[T::sfl(4, c, t)] = f4;
+    if (!valid) continue;
+    sflx[T::sfl(4, c, t)] = fma(-bsum, c2 / gm1, f4);
     if constexpr (DIR == 0) {
       if (pp.on) {
         const double dt = dt_pp > 0 ? dt_pp : z.dt_local[node_idx(0, c, f < 0 ? 0 : f)];
@@ -372,7 +406,7 @@ __global__ void __launch_bounds__(256) weno_mix_flux_diff(Zone z, double eps_ref
     if (cbase + c >= ncol_max || a > m - 1) continue;
     const int64_t iq = node_idx(0, c, a);
 #pragma unroll
-    for (int v = 0; v < T::NV; ++v) z.dq[iq + v * szq] -= sflx[T::sfl(v, c, t + 1)] - sflx[T::sfl(v, c, t)];
+    for (int v = 0; v < T::NV; ++v) red_add(z.dq + iq + v * szq, sflx[T::sfl(v, c, t)] - sflx[T::sfl(v, c, t + 1)]);
   }
 }
 

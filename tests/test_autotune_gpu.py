@@ -134,3 +134,28 @@ def test_viscous_forms_identical_and_in_parity(name):
         assert rel_err(out[v][1:], oz["dq"][1:], momentum=(0, 1, 2)) <= 1e-11, f"form {v}"
     var, ms = gz.ctx.viscous_variant()
     assert var == 2
+
+
+@pytest.mark.parametrize("scheme", [52, 72])
+@pytest.mark.parametrize("n, ny, nz", [(32, 7, 8), (33, 16, 9), (65, 31, 18), (121, 91, 79)])
+def test_untuned_air_tiles_by_block_size(scheme, n, ny, nz):
+    """A context that was neither tuned nor set picks its shapes by the
+    block's size: extents around the tile lengths (7, 15, 31), the last one on
+    the other side of the rule's line.  Bitwise the fluxes of a set variant,
+    and the oracle's at the single-call bar."""
+    case = cases.perturbed(cases.sine_wave(n=n, ny=ny, nz=nz, scheme=scheme, viscous=False, amp=0.2), seed=3, amp=0.1)
+    gz = GpuZone(case)
+    gz.initialize()
+    out = []
+    for v in (None, 0, 1):
+        gz.t["dq"].zero_()
+        if v is not None:
+            gz.ctx.set_tile_variants([v, v, v])
+        gz.ctx.inviscid()
+        out.append(gz.get("dq"))
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+    if n < 100:
+        oz = pyoracle.OracleZone(case)
+        oz.initialize()
+        oz.call("orc_compute_inviscid_flux")
+        assert rel_err(out[0], oz["dq"]) <= 1e-11
