@@ -509,6 +509,42 @@ int cfk_set_mechanism(cfk_ctx *c, const cfk_mechanism *m) {
     }
     kn.n_inv[r] = n;
   }
+  // species by the number of reactions that involve them, so that the lanes
+  // of a group, which take every third position, have like work
+  int uses[kMaxSpec] = {}, pos[kMaxSpec] = {};
+  for (int l = 0; l < ns; ++l) {
+    kn.order_sp[l] = (unsigned char)l;
+    for (int r = 0; r < m->n_reac; ++r) uses[l] += kn.inv_mask[r] >> l & 1u;
+  }
+  std::stable_sort(kn.order_sp, kn.order_sp + ns, [&](int x, int y) { return uses[x] > uses[y]; });
+  for (int i = 0; i < ns; ++i) pos[kn.order_sp[i]] = i;
+  kn.lists_ok = 1;
+  for (int r = 0; r < m->n_reac; ++r)
+    for (int l = 0; l < ns; ++l) {
+      const int f = m->stoi_f[r][l], b = m->stoi_b[r][l];
+      if (kn.n_f[r] + f > kMaxMol || kn.n_b[r] + b > kMaxMol) {
+        kn.lists_ok = 0;
+        continue;
+      }
+      for (int k = 0; k < f; ++k) kn.lf[r][kn.n_f[r]++] = (unsigned char)pos[l];
+      for (int k = 0; k < b; ++k) kn.lb[r][kn.n_b[r]++] = (unsigned char)pos[l];
+    }
+  // reactions of like type next to each other, so that the lanes of a warp
+  // diverge in few rounds of the deal
+  for (int r = 0; r < m->n_reac; ++r) kn.deal[r] = (unsigned char)r;
+  std::stable_sort(kn.deal, kn.deal + m->n_reac, [&](int x, int y) { return kn.type[x] > kn.type[y]; });
+  for (int i = 0; i < ns; ++i) {
+    const int l = kn.order_sp[i];
+    kn.ent_start[i] = (unsigned char)kn.n_ent;
+    for (int r = 0; r < m->n_reac; ++r) {
+      if (!(kn.inv_mask[r] >> l & 1u)) continue;
+      kn.ent_r[kn.n_ent] = (unsigned char)r;
+      kn.ent_f[kn.n_ent] = m->stoi_f[r][l];
+      kn.ent_b[kn.n_ent] = m->stoi_b[r][l];
+      ++kn.n_ent;
+    }
+  }
+  for (int i = ns; i <= kMaxSpec; ++i) kn.ent_start[i] = (unsigned char)kn.n_ent;
   CFK_CHECK(c, cudaSetDevice(c->hp.device), "cudaSetDevice");
   CFK_CHECK(c, cudaMemcpy(c->d_mech, &h, sizeof(Mech), cudaMemcpyHostToDevice), "mechanism upload");
   c->h_mech = h;

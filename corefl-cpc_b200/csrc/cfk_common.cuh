@@ -48,6 +48,18 @@ struct Zone {
   unsigned long long *inflow_draws;  // applications of a fluctuating inflow so far (context-owned counter)
 };
 
+// 1/x for x whose reciprocal is a normal number: the hardware's 20-bit
+// approximation (PTX rcp.approx.ftz.f64) and one third-order Householder step
+// y (1 + e + e^2), e = 1 - x y, whose remainder e^3 is below 2^-60; the result
+// is within 2 ulp.  Three FMAs, against a division sequence with its range
+// checks.  x = 0 and x = inf give NaN.
+__device__ __forceinline__ double rcp_nr(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
 // *p += v without waiting for *p: the addition is done at L2 (one rounding, as
 // a load, an add and a store have).  For right-hand sides that a launch adds
 // to once per node: the flux-difference phase then ends with its stores

@@ -273,84 +273,77 @@ __global__ void __launch_bounds__(128) wu_reaction_queue_kernel(Zone z, Param p,
 
 // ---------------------------------------------------------------------------
 // Compile-time species count (NS = 9, the bundled H2 mechanisms): the same
-// two schedules over zero_d_substep_ns, with each lane's NS x NS system in
-// shared memory.
+// two schedules with a group of kGroupLanes lanes a node (chem_fast.cuh).
+// Both take their nodes with the same code below, so they are bit-identical.
+// Bound by latency and instruction issue (IPC 1.5 an SM, FP64 pipe 20 %): 168
+// registers, three CTAs an SM; four CTAs at 128 registers spill 270 bytes and
+// were slower (33.1 against 32.3 ms on 2^20 reactors, at an earlier step).
 // ---------------------------------------------------------------------------
-constexpr int kFastBlock = 64;
+constexpr int kGroupBlock = 128, kGroupCtas = 3, kGroupLanes = 3;
 
-template <int NS>
-__host__ __device__ constexpr int fast_smem_bytes() { return (NS * NS + NS) * kFastBlock * (int)sizeof(double); }
+template <int NS, int GL>
+struct GroupSmem {
+  static constexpr int kNodes = kGroupBlock / 32 * (32 / GL);  // groups a CTA
+  GroupTables<NS> tb;
+  GroupMem<NS> mem[kNodes];
+};
 
-template <int NS>
-__global__ void __launch_bounds__(kFastBlock) wu_reaction_plain_ns_kernel(Zone z, Param p,
-                                                                         const __grid_constant__ Mech mech, double dt,
-                                                                         int *nsub_out, int *err) {
-  const Mech *mc = &mech;
-  extern __shared__ double sys[];
-  const LaneSlot L{sys + threadIdx.x, kFastBlock}, R{sys + NS * NS * kFastBlock + threadIdx.x, kFastBlock};
-  const Dims d = z.d;
-  const long long q = (long long)blockIdx.x * kFastBlock + threadIdx.x;
-  if (q >= (long long)d.mx * d.my * d.mz) return;
-  const int i = (int)(q % d.mx), rem = (int)(q / d.mx), j = rem % d.my, k = rem / d.my;
-  const int64_t id = d.idx(d.ngg, i, j, k), iq = d.idx(0, i, j, k);
-  NodeStateN<NS> s;
-  double yk[NS], pres;
-  load_node_ns<NS>(z, id, iq, s, yk, pres);
-  int n_sub;
-  double h, h_last;
-  bool capped;
-  substep_plan(dt, s.ts, n_sub, h, h_last, capped);
-  if (capped) atomicOr(err, 2);
-  bool ok = true;
-  for (int n = 0; n < n_sub; ++n) ok &= zero_d_substep_ns<NS>(mc, p.chem_advance_method, h, s, yk, pres, L, R);
-  int taken = n_sub;
-  if (abs(h_last) > 1e-12) {
-    ok &= zero_d_substep_ns<NS>(mc, p.chem_advance_method, h_last, s, yk, pres, L, R);
-    ++taken;
+// QUEUE: persistent; a group whose node is finished writes it back and takes
+// the next one from a global counter (one atomicAdd per warp, shared out among
+// its groups), so nodes with uneven substep counts do not leave the rest of
+// the warp idle.  With a node list, the queue runs over list[0 ..
+// *list_count) instead of all nodes.  Otherwise group i takes node i.
+template <int NS, int GL, bool QUEUE>
+__global__ void __launch_bounds__(kGroupBlock, kGroupCtas)
+    wu_reaction_ns_kernel(Zone z, Param p, const __grid_constant__ Mech mech, double dt, int *nsub_out, int *err,
+                          unsigned int *counter, const unsigned int *list, const unsigned int *list_count) {
+  extern __shared__ __align__(16) unsigned char group_raw[];
+  using SM = GroupSmem<NS, GL>;
+  SM &sm = *reinterpret_cast<SM *>(group_raw);
+  load_group_tables<NS>(sm.tb, mech, threadIdx.x, kGroupBlock);
+  for (int e = threadIdx.x; e < SM::kNodes; e += kGroupBlock) {
+    sm.mem[e].g[NS] = 0.0;
+    sm.mem[e].act[NS] = 1.0;
   }
-  if (!ok) atomicOr(err, 1);
-  store_node_ns<NS>(z, p.n_scalar, id, s, yk, pres);
-  if (nsub_out) nsub_out[iq] = taken;
-}
-
-// Work-queue schedule (see wu_reaction_queue_kernel), optionally over a node list.
-template <int NS>
-__global__ void __launch_bounds__(kFastBlock) wu_reaction_queue_ns_kernel(Zone z, Param p,
-                                                                         const __grid_constant__ Mech mech, double dt,
-                                                                         int *nsub_out, int *err,
-                                                                         unsigned int *counter,
-                                                                         const unsigned int *list,
-                                                                         const unsigned int *list_count) {
-  const Mech *mc = &mech;
-  extern __shared__ double sys[];
-  const LaneSlot L{sys + threadIdx.x, kFastBlock}, R{sys + NS * NS * kFastBlock + threadIdx.x, kFastBlock};
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const Lane<NS, GL> me(mech, lane);
+  const int slot = (threadIdx.x >> 5) * (32 / GL) + me.base / GL;
+  GroupMem<NS> &S = sm.mem[slot];
   const Dims d = z.d;
   const unsigned int total = list ? *list_count : (unsigned int)d.mx * d.my * d.mz;
-  const int lane = threadIdx.x & 31;
-  NodeStateN<NS> s;
-  double yk[NS], pres = 0, h = 0, h_last = 0;
+  const int n_reac = mech.kn.n_reac, method = p.chem_advance_method;
+  GroupState<NS / GL> s = {};
+  s.T = 1000.0; s.q[0] = 1.0; s.iJac = 1.0;  // a state that computes, for the groups without a node
+#pragma unroll
+  for (int k = 0; k < NS / GL; ++k) s.rY[k] = 1.0;
+  double h = 0, h_last = 0;
   int n_sub = 0, done = 0, taken = 0;
-  int64_t id = 0, iq = 0;
-  bool ok = true, have = false, exhausted = false;
+  int64_t id = 0;
+  bool ok = true, have = false, exhausted = !me.own;
   for (;;) {
     const bool need = !have && !exhausted;
-    const unsigned int mask = __ballot_sync(0xffffffffu, need);
+    const unsigned int mask = __ballot_sync(0xffffffffu, need && me.j == 0);  // one lane a group asks
     if (mask) {
-      unsigned int base = 0;
-      const int leader = __ffs(mask) - 1;
-      if (lane == leader) base = atomicAdd(counter, (unsigned int)__popc(mask));
-      base = __shfl_sync(0xffffffffu, base, leader);
+      unsigned int node;
+      if (QUEUE) {
+        unsigned int first = 0;
+        const int leader = __ffs(mask) - 1;
+        if (lane == leader) first = atomicAdd(counter, (unsigned int)__popc(mask));
+        first = __shfl_sync(0xffffffffu, first, leader);
+        node = first + __popc(mask & ((1u << me.base) - 1));
+      } else {
+        node = blockIdx.x * SM::kNodes + slot;
+      }
       if (need) {
-        unsigned int node = base + __popc(mask & ((1u << lane) - 1));
         if (node < total) {
           if (list) node = list[node];
           const int i = node % d.mx, rem = node / d.mx, j = rem % d.my, k = rem / d.my;
           id = d.idx(d.ngg, i, j, k);
-          iq = d.idx(0, i, j, k);
-          load_node_ns<NS>(z, id, iq, s, yk, pres);
+          load_group<NS, GL>(z, id, d.idx(0, i, j, k), me, s);
           bool capped;
           substep_plan(dt, s.ts, n_sub, h, h_last, capped);
-          if (capped) atomicOr(err, 2);
+          if (capped && me.j == 0) atomicOr(err, 2);
           done = 0;
           taken = 0;
           ok = true;
@@ -358,37 +351,39 @@ __global__ void __launch_bounds__(kFastBlock) wu_reaction_queue_ns_kernel(Zone z
         } else {
           exhausted = true;
         }
+        if (!QUEUE) exhausted = true;
       }
     }
     if (!__any_sync(0xffffffffu, have)) break;
-    if (have) {
-      const double hh = done < n_sub ? h : h_last;
-      const bool run = done < n_sub || abs(h_last) > 1e-12;
-      if (run) {
-        ok &= zero_d_substep_ns<NS>(mc, p.chem_advance_method, hh, s, yk, pres, L, R);
-        ++taken;
-      }
-      ++done;
-      if (done > n_sub) {
-        if (!ok) atomicOr(err, 1);
-        store_node_ns<NS>(z, p.n_scalar, id, s, yk, pres);
-        if (nsub_out) nsub_out[iq] = taken;
-        have = false;
-      }
+    // substeps 0..n_sub-1 use h, the last one h_last (skipped if ~0)
+    const double hh = done < n_sub ? h : h_last;
+    const bool run = have && (done < n_sub || abs(h_last) > 1e-12);
+    if (__any_sync(0xffffffffu, run)) ok &= group_substep<NS, GL>(z, sm.tb, S, me, n_reac, method, hh, run, s);
+    if (run) ++taken;
+    if (have && ++done > n_sub) {
+      if (!ok && me.j == 0) atomicOr(err, 1);
+      store_group<NS, GL>(z, p.n_scalar, id, me, s);
+      if (nsub_out && me.j == 0) nsub_out[s.iq] = taken;
+      have = false;
     }
   }
 }
 
-// Persistent grid of the work-queue kernels: resident blocks per SM x SMs.
-template <class K>
-static long long queue_blocks(K kernel, int block, int smem, int n_sm, long long nodes) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  long long blocks = (long long)n_sm * per_sm;
-  const long long need = (nodes + block - 1) / block;
-  if (blocks > need) blocks = need;
-  return blocks < 1 ? 1 : blocks;
+template <bool QUEUE>
+static cudaError_t launch_group_kernel(const Zone &z, const Param &p, const Mech &mech, double dt, int *nsub_out,
+                                       int *err, unsigned int *counter, const unsigned int *list,
+                                       const unsigned int *list_count, long long nodes, int n_sm, cudaStream_t st) {
+  constexpr int smem = (int)sizeof(GroupSmem<kMaxSpec, kGroupLanes>),
+                per_cta = GroupSmem<kMaxSpec, kGroupLanes>::kNodes;
+  cudaError_t e = cudaFuncSetAttribute(wu_reaction_ns_kernel<kMaxSpec, kGroupLanes, QUEUE>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  long long blocks = (nodes + per_cta - 1) / per_cta;
+  if (QUEUE && blocks > (long long)n_sm * kGroupCtas) blocks = (long long)n_sm * kGroupCtas;
+  if (blocks < 1) blocks = 1;
+  wu_reaction_ns_kernel<kMaxSpec, kGroupLanes, QUEUE><<<(unsigned)blocks, kGroupBlock, smem, st>>>(
+      z, p, mech, dt, nsub_out, err, counter, list, list_count);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_finite_rate_chemistry(const Zone &z, const Mech *mc, cudaStream_t st) {
@@ -400,19 +395,12 @@ cudaError_t launch_wu_reaction(const Zone &z, const Param &p, const Mech *mc, co
                                int schedule, int *nsub_out, int *err, unsigned int *counter, int n_sm,
                                cudaStream_t st) {
   const long long total = (long long)z.d.mx * z.d.my * z.d.mz;
-  if (p.n_spec == kMaxSpec) {
-    constexpr int smem = fast_smem_bytes<kMaxSpec>();
-    if (schedule == 0) {
-      wu_reaction_plain_ns_kernel<kMaxSpec><<<(unsigned)((total + kFastBlock - 1) / kFastBlock), kFastBlock, smem, st>>>(
-          z, p, mc_host, dt, nsub_out, err);
-    } else {
-      cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
-      if (e != cudaSuccess) return e;
-      const long long blocks = queue_blocks(wu_reaction_queue_ns_kernel<kMaxSpec>, kFastBlock, smem, n_sm, total);
-      wu_reaction_queue_ns_kernel<kMaxSpec><<<(unsigned)blocks, kFastBlock, smem, st>>>(
-          z, p, mc_host, dt, nsub_out, err, counter, nullptr, nullptr);
-    }
-    return cudaGetLastError();
+  if (p.n_spec == kMaxSpec && mc_host.kn.lists_ok) {
+    if (schedule == 0)
+      return launch_group_kernel<false>(z, p, mc_host, dt, nsub_out, err, nullptr, nullptr, nullptr, total, n_sm, st);
+    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
+    if (e != cudaSuccess) return e;
+    return launch_group_kernel<true>(z, p, mc_host, dt, nsub_out, err, counter, nullptr, nullptr, total, n_sm, st);
   }
   if (schedule == 0) {
     wu_reaction_plain_kernel<<<dim3((z.d.mx + 127) / 128, z.d.my, z.d.mz), 128, 0, st>>>(z, p, mc, dt, nsub_out, err);
@@ -434,13 +422,8 @@ cudaError_t launch_wu_reaction_list(const Zone &z, const Param &p, const Mech *m
                                     int *err, unsigned int *counter, int n_sm, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
   if (e != cudaSuccess) return e;
-  if (p.n_spec == kMaxSpec) {
-    constexpr int smem = fast_smem_bytes<kMaxSpec>();
-    const long long blocks = queue_blocks(wu_reaction_queue_ns_kernel<kMaxSpec>, kFastBlock, smem, n_sm, max_nodes);
-    wu_reaction_queue_ns_kernel<kMaxSpec><<<(unsigned)blocks, kFastBlock, smem, st>>>(z, p, mc_host, dt, nullptr, err,
-                                                                                    counter, list, list_count);
-    return cudaGetLastError();
-  }
+  if (p.n_spec == kMaxSpec && mc_host.kn.lists_ok)
+    return launch_group_kernel<true>(z, p, mc_host, dt, nullptr, err, counter, list, list_count, max_nodes, n_sm, st);
   long long blocks = (long long)n_sm * 8;
   const long long need = (max_nodes + 127) / 128;
   if (blocks > need) blocks = need;

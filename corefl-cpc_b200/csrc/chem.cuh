@@ -15,6 +15,7 @@
 namespace cfk {
 
 constexpr int kMaxReac = 24;
+constexpr int kMaxMol = 3;       // molecules on one side of a reaction (species lists of the lane-group kernels)
 constexpr int kMaxInvolved = 6;  // distinct species appearing in one reaction
 
 struct Kinetics {
@@ -32,6 +33,20 @@ struct Kinetics {
   // (net_mask), for loops whose species index is a compile-time constant
   signed char stf[kMaxReac][kMaxSpec], stb[kMaxReac][kMaxSpec];
   unsigned int inv_mask[kMaxReac], net_mask[kMaxReac];
+  // the same again for the lane-group kernels (chem_fast.cuh), species by
+  // their position in `order_sp` (the most involved first) and all factors as
+  // doubles: the reactants and products of a reaction, one entry a molecule
+  // (lists_ok = 0 where a side has more than kMaxMol of them); the reactions
+  // in the order they are dealt to the lanes; and, position by position, the
+  // reactions that involve the species
+  int lists_ok;
+  unsigned char order_sp[kMaxSpec];
+  unsigned char n_f[kMaxReac], n_b[kMaxReac], lf[kMaxReac][kMaxMol], lb[kMaxReac][kMaxMol];
+  unsigned char deal[kMaxReac];
+  int n_ent;
+  unsigned char ent_start[kMaxSpec + 1];
+  unsigned char ent_r[kMaxReac * kMaxInvolved];
+  double ent_f[kMaxReac * kMaxInvolved], ent_b[kMaxReac * kMaxInvolved];
 };
 
 // Mixture and mechanism tables in one device block.

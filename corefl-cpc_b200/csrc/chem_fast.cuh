@@ -1,23 +1,26 @@
-// Point-implicit reaction substep with the species count fixed at compile
-// time.  Same model and, term by term, the same arithmetic order as the
-// runtime-count path in chem.cu/chem.cuh (reference
-// src/FiniteRateChem.cu:1466-1822, src/StrangSplitting.cu:43-224), laid out
-// for the GPU:
-//  * every per-species quantity is a register array indexed by compile-time
-//    constants; a reaction's species are selected with the uniform bit masks
-//    of the dense stoichiometry tables (all lanes process the same reaction,
-//    so these branches never diverge);
-//  * rates of progress are consumed as soon as they are formed: sources,
-//    destruction rates and the Jacobian are accumulated reaction by reaction
-//    (each accumulator still sums the reactions in mechanism order);
-//  * the NS x NS system matrix and right-hand side live in shared memory,
-//    entry e of lane t at base[e * stride + t], so the Jacobian's sparse
-//    accumulation and the pivoted LU's runtime row indices address shared
-//    memory rather than local memory;
-//  * the mechanism tables are a __grid_constant__ kernel parameter: uniform
-//    reads through the constant cache;
-//  * divisions by the same value are one reciprocal and products, so results
-//    match the runtime-count path to rounding, not bit for bit.
+// Point-implicit reaction substep by a group of GL = 3 lanes, NS / GL species
+// a lane (ten nodes a warp).  The same model as the runtime-count path in
+// chem.cu/chem.cuh (reference src/FiniteRateChem.cu:1466-1822,
+// src/StrangSplitting.cu:43-224).  A node's substeps are a serial chain, so
+// what counts is the instructions of a substep, its latency, and how many
+// warps hide it:
+//  * the lanes share the reactions (rates), the species (thermodynamics) and
+//    the columns of the matrix;
+//  * a rate of progress is kf' times the product of a_k = c_k exp(g_k) over
+//    the reactants or the products, kf' = A T^b exp(-Ea/T - sum of the
+//    reactants' g_k): with one exponential a species, the equilibrium constant
+//    costs a reaction no exponential and no division;
+//  * the matrix is in molar units (rows and columns scaled by the molar
+//    masses), in which its diagonal is mostly the largest entry of its column,
+//    and is solved by Gauss-Jordan elimination with threshold pivoting in
+//    registers, three columns a lane, the multipliers passed on by shuffles;
+//  * the mechanism tables are in shared memory, every factor a double.
+// Lanes a node, measured on 2^20 H2/air reactors of 4-64 substeps each and on
+// 1021 of them (ms): one, with the matrix in its registers, 31.9 and 2.72 (255
+// registers, 8 warps an SM, 80 000 cycles a substep); nine, a row each, 52.6
+// and 0.73 (a node takes four times the instructions); three, 26.0 and 0.71.
+// One lane with the matrix in shared memory, before, took 49.7 and 4.54.
+// Results match the runtime-count path to rounding.
 #pragma once
 
 #include "chem.cuh"
@@ -38,350 +41,438 @@ __device__ __forceinline__ void enthalpy_cp_one(const Thermo *th, int i, double 
 
 template <int NS>
 __device__ __forceinline__ void enthalpy_cp_ns(const Thermo *th, double t, double *h, double *cp) {
-  const double t2 = t * t, t3 = t2 * t, t4 = t3 * t, t5 = t4 * t;
 #pragma unroll
-  for (int i = 0; i < NS; ++i) {
-    if (t < th->t_low[i] || t > th->t_high[i]) {
-      const bool lo = t < th->t_low[i];
-      const double tt = lo ? th->t_low[i] : th->t_high[i];
-      const double *c = lo ? th->low[i] : th->high[i];
-      const double tt2 = tt * tt, tt3 = tt2 * tt, tt4 = tt3 * tt, tt5 = tt4 * tt;
-      h[i] = c[0] * tt + 0.5 * c[1] * tt2 + c[2] * tt3 / 3 + 0.25 * c[3] * tt4 + 0.2 * c[4] * tt5 + c[5];
-      cp[i] = c[0] + c[1] * tt + c[2] * tt2 + c[3] * tt3 + c[4] * tt4;
-      h[i] += cp[i] * (t - tt);
-    } else {
-      const double *c = t < th->t_mid[i] ? th->low[i] : th->high[i];
-      h[i] = c[0] * t + 0.5 * c[1] * t2 + c[2] * t3 / 3 + 0.25 * c[3] * t4 + 0.2 * c[4] * t5 + c[5];
-      cp[i] = c[0] + c[1] * t + c[2] * t2 + c[3] * t3 + c[4] * t4;
-    }
-    h[i] *= th->gas_const[i];
-    cp[i] *= th->gas_const[i];
-  }
+  for (int i = 0; i < NS; ++i) enthalpy_cp_one(th, i, t, h[i], cp[i]);
 }
 
+// G_i / (R T), held at the end of the species' range outside it.
+__device__ __forceinline__ double gibbs_one(const double *low, const double *high, double t_low, double t_mid,
+                                            double t_high, double t, double lnT, double iT) {
+  const double *c = t < t_mid ? low : high;
+  double tt = t, ln = lnT, it = iT;
+  if (t < t_low || t > t_high) {
+    tt = t < t_low ? t_low : t_high;
+    ln = log(tt);
+    it = 1.0 / tt;
+  }
+  const double p = fma(tt, fma(tt, fma(tt, 0.05 * c[4], (1.0 / 12) * c[3]), (1.0 / 6) * c[2]), 0.5 * c[1]);
+  return fma(c[0], 1.0 - ln, fma(c[5], it, fma(-tt, p, -c[6])));
+}
+
+// Mechanism tables of a CTA in shared memory, species by position.
 template <int NS>
-__device__ __forceinline__ bool temperature_newton_ns(const Thermo *th, const double *yk, double total_energy,
-                                                      double rho, double V2, double &t, double &p) {
-  double gas_const = 0;
-#pragma unroll
-  for (int l = 0; l < NS; ++l) gas_const += yk[l] * th->gas_const[l];
-  const double e = total_energy / rho - 0.5 * V2;
-  double err = 1;
-  int iter = 0;
-  while (err > 1e-5 && iter++ < 1000) {
-    double h_i[NS], cp_i[NS];
-    enthalpy_cp_ns<NS>(th, t, h_i, cp_i);
-    double cp_tot = 0, h = 0;
-#pragma unroll
-    for (int l = 0; l < NS; ++l) {
-      cp_tot += cp_i[l] * yk[l];
-      h += h_i[l] * yk[l];
-    }
-    const double e_t = h - gas_const * t;
-    const double cv = cp_tot - gas_const;
-    const double t1 = t - (e_t - e) / cv;
-    err = abs(1 - t1 / t);
-    t = t1;
-  }
-  p = rho * t * gas_const;
-  return err <= 1e-5;
-}
-
-template <int NS>
-__device__ __forceinline__ void gibbs_ns(const Thermo *th, double t, double lnT, double iT, double *g) {
-  const double t2 = t * t, t3 = t2 * t, t4 = t3 * t;
-#pragma unroll
-  for (int i = 0; i < NS; ++i) {
-    if (t < th->t_low[i] || t > th->t_high[i]) {
-      const bool lo = t < th->t_low[i];
-      const double tt = lo ? th->t_low[i] : th->t_high[i];
-      const double *c = lo ? th->low[i] : th->high[i];
-      const double tt2 = tt * tt, tt3 = tt2 * tt, tt4 = tt3 * tt;
-      g[i] = c[0] * (1.0 - log(tt)) - 0.5 * c[1] * tt - c[2] * tt2 / 6.0 - c[3] * tt3 / 12.0 - c[4] * tt4 * 0.05 +
-             c[5] / tt - c[6];
-    } else {
-      const double *c = t < th->t_mid[i] ? th->low[i] : th->high[i];
-      g[i] = c[0] * (1.0 - lnT) - 0.5 * c[1] * t - c[2] * t2 / 6.0 - c[3] * t3 / 12.0 - c[4] * t4 * 0.05 + c[5] * iT -
-             c[6];
-    }
-  }
-}
-
-// A per-lane slot in shared memory: entry e at p[e * stride].
-struct LaneSlot {
-  double *p;
-  int stride;
-  __device__ __forceinline__ double &operator()(int e) const { return p[e * stride]; }
+struct GroupTables {
+  static constexpr int LD = (NS + 1) / 2 * 2;  // rows start on 16 bytes
+  double net[kMaxReac][LD];                    // net stoichiometry of reaction r
+  double tb[kMaxReac][LD];                     // third-body efficiencies
+  double low[NS][7], high[NS][7], imw3[LD];    // imw3: 1e-3 / W (mol/cm^3 of kg/m^3)
+  double A[kMaxReac], b[kMaxReac], Ea[kMaxReac], A2[kMaxReac], b2[kMaxReac], Ea2[kMaxReac];
+  double troe_alpha[kMaxReac], troe_it3[kMaxReac], troe_it1[kMaxReac], troe_t2[kMaxReac];
+  double ent_f[kMaxReac * kMaxInvolved], ent_b[kMaxReac * kMaxInvolved];
+  int type[kMaxReac], order[kMaxReac];
+  uint2 mol[kMaxReac];  // positions of the reactants and products, a byte each; NS stands for none
+  unsigned char deal[kMaxReac];
+  unsigned char ent_r[kMaxReac * kMaxInvolved];
 };
 
-// Column-pivoted LU solve of L x = R in the elimination order of
-// solve_chem_system (divisions by a pivot as one reciprocal each); L and R
-// are overwritten, x returned in registers.
+// A group's own shared memory.  Its size is 6 words past a multiple of 32, so
+// that the ten groups of a warp, which read the same entry or three adjacent
+// ones, hit different banks.
 template <int NS>
-__device__ __forceinline__ void lu_solve_ns(const LaneSlot &L, const LaneSlot &R, double *x) {
-  int ipiv[NS];
-  double rdiag[NS];
-#pragma unroll
-  for (int n = 0; n < NS; ++n) {
-    int ik = n;
-#pragma unroll
-    for (int m = n; m < NS; ++m) {
-      double v = L(m * NS + n);
-#pragma unroll
-      for (int t = 0; t < n; ++t) v -= L(m * NS + t) * L(t * NS + n);
-      L(m * NS + n) = v;
-      if (abs(v) > abs(L(ik * NS + n))) ik = m;
-    }
-    ipiv[n] = ik;
-    if (ik != n) {
-#pragma unroll
-      for (int t = 0; t < NS; ++t) {
-        const double mid = L(ik * NS + t);
-        L(ik * NS + t) = L(n * NS + t);
-        L(n * NS + t) = mid;
-      }
-    }
-#pragma unroll
-    for (int p = n + 1; p < NS; ++p) {
-      double v = L(n * NS + p);
-#pragma unroll
-      for (int t = 0; t < n; ++t) v -= L(n * NS + t) * L(t * NS + p);
-      L(n * NS + p) = v;
-    }
-    rdiag[n] = 1.0 / L(n * NS + n);
-#pragma unroll
-    for (int m = n + 1; m < NS; ++m) L(m * NS + n) *= rdiag[n];
-  }
-#pragma unroll
-  for (int m = 0; m < NS; ++m) {
-    const int t = ipiv[m];
-    if (t != m) {
-      const double mid = R(t);
-      R(t) = R(m);
-      R(m) = mid;
-    }
-  }
-#pragma unroll
-  for (int m = 0; m < NS; ++m) x[m] = R(m);
-#pragma unroll
-  for (int m = 1; m < NS; ++m)
-#pragma unroll
-    for (int t = 0; t < m; ++t) x[m] -= L(m * NS + t) * x[t];
-  x[NS - 1] *= rdiag[NS - 1];
-#pragma unroll
-  for (int m = NS - 2; m >= 0; --m) {
-#pragma unroll
-    for (int t = m + 1; t < NS; ++t) x[m] -= L(m * NS + t) * x[t];
-    x[m] *= rdiag[m];
-  }
-}
-
-template <int NS>
-struct NodeStateN {
-  double q[5];
-  double rY[NS];
-  double T;
-  double cn[5], cnY[NS];
-  double iJac;
-  double ts;  // reaction time scale
+struct GroupMem {
+  double c[NS], w[NS];
+  double g[NS + 1], act[NS + 1];      // entry NS: no molecule (g 0, activity 1)
+  double q1[kMaxReac], q2[kMaxReac];  // rates of progress
+  static constexpr int kUsed = 4 * NS + 2 + 2 * kMaxReac;
+  double pad[((3 - kUsed) % 16 + 16) % 16];
 };
 
 template <int NS>
-__device__ __forceinline__ void load_node_ns(const Zone &z, int64_t id, int64_t iq, NodeStateN<NS> &s, double *yk,
-                                             double &pres) {
-  const int64_t sz = z.d.plane(z.d.ngg), szq = z.d.plane(0);
-#pragma unroll
-  for (int l = 0; l < 5; ++l) s.q[l] = z.cv[id + l * sz];
-#pragma unroll
-  for (int l = 0; l < NS; ++l) {
-    s.rY[l] = z.cv[id + (5 + l) * sz];
-    yk[l] = z.sv[id + l * sz];
+__device__ __forceinline__ void load_group_tables(GroupTables<NS> &tb, const Mech &m, int tid, int nt) {
+  const Kinetics &kn = m.kn;
+  for (int e = tid; e < NS * 7; e += nt) {
+    const int sp = kn.order_sp[e / 7];
+    tb.low[e / 7][e % 7] = m.th.low[sp][e % 7];
+    tb.high[e / 7][e % 7] = m.th.high[sp][e % 7];
   }
-  s.T = z.bv[id + 5 * sz];
-  pres = z.bv[id + 4 * sz];
-  if (z.Cn) {
-#pragma unroll
-    for (int l = 0; l < 5; ++l) s.cn[l] = z.Cn[iq + l * szq];
-#pragma unroll
-    for (int l = 0; l < NS; ++l) s.cnY[l] = z.Cn[iq + (5 + l) * szq];
-  } else {
-#pragma unroll
-    for (int l = 0; l < 5; ++l) s.cn[l] = 0;
-#pragma unroll
-    for (int l = 0; l < NS; ++l) s.cnY[l] = 0;
+  for (int i = tid; i < NS; i += nt) tb.imw3[i] = m.th.imw[kn.order_sp[i]] * 1e-3;
+  for (int r = tid; r < kMaxReac; r += nt) {
+    tb.A[r] = kn.A[r]; tb.b[r] = kn.b[r]; tb.Ea[r] = kn.Ea[r];
+    tb.A2[r] = kn.A2[r]; tb.b2[r] = kn.b2[r]; tb.Ea2[r] = kn.Ea2[r];
+    tb.troe_alpha[r] = kn.troe_alpha[r]; tb.troe_it3[r] = 1.0 / kn.troe_t3[r];
+    tb.troe_it1[r] = 1.0 / kn.troe_t1[r]; tb.troe_t2[r] = kn.troe_t2[r];
+    tb.type[r] = kn.type[r]; tb.order[r] = kn.order[r];
+    tb.deal[r] = kn.deal[r];
+    unsigned f = 0, b = 0;
+    for (int k = 0; k < kMaxMol; ++k) {
+      f |= (k < kn.n_f[r] ? (unsigned)kn.lf[r][k] : (unsigned)NS) << 8 * k;
+      b |= (k < kn.n_b[r] ? (unsigned)kn.lb[r][k] : (unsigned)NS) << 8 * k;
+    }
+    tb.mol[r] = make_uint2(f, b);
+    for (int i = 0; i < NS; ++i) {
+      const int sp = kn.order_sp[i];
+      tb.net[r][i] = (double)kn.stb[r][sp] - (double)kn.stf[r][sp];
+      tb.tb[r][i] = kn.tb[r][sp];
+    }
   }
-  s.iJac = 1.0 / z.jac[id];
-  s.ts = z.reaction_timeScale[id];
+  for (int e = tid; e < kn.n_ent; e += nt) {
+    tb.ent_f[e] = kn.ent_f[e]; tb.ent_b[e] = kn.ent_b[e];
+    tb.ent_r[e] = kn.ent_r[e];
+  }
 }
 
-template <int NS>
-__device__ __forceinline__ void store_node_ns(const Zone &z, int n_scalar, int64_t id, const NodeStateN<NS> &s,
-                                              const double *yk, double pres) {
+// A lane's place: lane j of its group, whose first lane is base; its slot k is
+// position k GL + j.  Lanes beyond the last group own nothing (own = false):
+// they read the last group's memory and write none.
+template <int NS, int GL>
+struct Lane {
+  static constexpr int SPL = NS / GL;
+  int j, base;
+  bool own;
+  int sp[SPL];                // species of the lane's slots
+  double mw[SPL], R[SPL];
+  double t_low[SPL], t_mid[SPL], t_high[SPL];
+  int ent[SPL], ent_end[SPL];
+  __device__ Lane(const Mech &m, int lane) {
+    constexpr int per = 32 / GL;
+    own = lane < per * GL;
+    const int grp = own ? lane / GL : per - 1;
+    base = grp * GL;
+    j = (lane - base) % GL;
+#pragma unroll
+    for (int k = 0; k < SPL; ++k) {
+      const int i = k * GL + j;
+      sp[k] = m.kn.order_sp[i];
+      mw[k] = m.th.mw[sp[k]]; R[k] = m.th.gas_const[sp[k]];
+      t_low[k] = m.th.t_low[sp[k]]; t_mid[k] = m.th.t_mid[sp[k]]; t_high[k] = m.th.t_high[sp[k]];
+      ent[k] = m.kn.ent_start[i];
+      ent_end[k] = m.kn.ent_start[i + 1];
+    }
+  }
+  // Sum over the group, in the same order in every lane.
+  __device__ double sum(double v) const {
+    double a = __shfl_sync(0xffffffffu, v, base);
+#pragma unroll
+    for (int k = 1; k < GL; ++k) a = __dadd_rn(a, __shfl_sync(0xffffffffu, v, base + k));
+    return a;
+  }
+  __device__ double min(double v) const {
+    double a = v;
+#pragma unroll
+    for (int k = 0; k < GL; ++k) a = fmin(a, __shfl_sync(0xffffffffu, v, base + k));
+    return a;
+  }
+};
+
+// State of a node across its substeps: the lane's species, the rest the same
+// in all lanes of the group.
+template <int SPL>
+struct GroupState {
+  double q[5], T, pres, iJac, ts;  // ts: reaction time scale
+  double rY[SPL], Y[SPL];
+  int64_t iq;  // the node in Cn
+};
+
+template <int NS, int GL>
+__device__ __forceinline__ void load_group(const Zone &z, int64_t id, int64_t iq, const Lane<NS, GL> &me,
+                                           GroupState<NS / GL> &s) {
   const int64_t sz = z.d.plane(z.d.ngg);
 #pragma unroll
-  for (int l = 0; l < 5; ++l) z.cv[id + l * sz] = s.q[l];
+  for (int k = 0; k < 5; ++k) s.q[k] = z.cv[id + k * sz];
 #pragma unroll
-  for (int l = 0; l < NS; ++l) {
-    z.cv[id + (5 + l) * sz] = s.rY[l];
-    z.sv[id + l * sz] = yk[l];
+  for (int k = 0; k < NS / GL; ++k) {
+    s.rY[k] = z.cv[id + (5 + me.sp[k]) * sz];
+    s.Y[k] = z.sv[id + me.sp[k] * sz];
   }
-  const double rho_inv = 1.0 / s.q[0];
-  for (int l = NS; l < n_scalar; ++l) z.sv[id + l * sz] = z.cv[id + (5 + l) * sz] * rho_inv;
-  z.bv[id] = s.q[0];
-  z.bv[id + sz] = s.q[1] * rho_inv;
-  z.bv[id + 2 * sz] = s.q[2] * rho_inv;
-  z.bv[id + 3 * sz] = s.q[3] * rho_inv;
-  z.bv[id + 4 * sz] = pres;
-  z.bv[id + 5 * sz] = s.T;
-  z.reaction_timeScale[id] = s.ts;
+  s.T = z.bv[id + 5 * sz];
+  s.pres = z.bv[id + 4 * sz];
+  s.iJac = 1.0 / z.jac[id];
+  s.ts = z.reaction_timeScale[id];
+  s.iq = iq;
 }
 
-// One substep of wu_zeroDReaction (methods 0 and 1).
-template <int NS>
-__device__ __forceinline__ bool zero_d_substep_ns(const Mech *mc, int method, double dt, NodeStateN<NS> &s,
-                                                  double *yk, double &pres, const LaneSlot &L, const LaneSlot &R) {
-  const Thermo *th = &mc->th;
-  const Kinetics &kn = mc->kn;
-  double c[NS];
+template <int NS, int GL>
+__device__ __forceinline__ void store_group(const Zone &z, int n_scalar, int64_t id, const Lane<NS, GL> &me,
+                                            const GroupState<NS / GL> &s) {
+  const int64_t sz = z.d.plane(z.d.ngg);
 #pragma unroll
-  for (int l = 0; l < NS; ++l) c[l] = s.rY[l] * th->imw[l] * 1e-3;
-  const double t = s.T, lnT = log(t), iT = 1.0 / t;
-  double g[NS];
-  gibbs_ns<NS>(th, t, lnT, iT, g);
-  constexpr double temp_p = 101325.0 / kRu * 1e-3;  // mol K / cm^3
-  const double temp_t = temp_p * iT;
-  double creation[NS], omega_d[NS];
-#pragma unroll
-  for (int l = 0; l < NS; ++l) { creation[l] = 0; omega_d[l] = 0; }
-  if (method == 1) {
-#pragma unroll
-    for (int e = 0; e < NS * NS; ++e) L(e) = 0;
+  for (int k = 0; k < NS / GL; ++k) {
+    z.cv[id + (5 + me.sp[k]) * sz] = s.rY[k];
+    z.sv[id + me.sp[k] * sz] = s.Y[k];
   }
-  for (int r = 0; r < kn.n_reac; ++r) {
-    const int type = kn.type[r];
-    const unsigned inv = kn.inv_mask[r];
-    double kf = kn.A[r] * exp(kn.b[r] * lnT - kn.Ea[r] * iT);
-    double cc = 0;
-    if (type > 3) {
+  const double rho_inv = 1.0 / s.q[0];
+  if (me.j == 0) {
 #pragma unroll
-      for (int l = 0; l < NS; ++l) cc += c[l] * kn.tb[r][l];
-    }
-    if (type == 3) {
-      kf += kn.A2[r] * exp(kn.b2[r] * lnT - kn.Ea2[r] * iT);
-    } else if (type == 4) {
+    for (int k = 0; k < 5; ++k) z.cv[id + k * sz] = s.q[k];
+    z.reaction_timeScale[id] = s.ts;
+  } else if (me.j == 1) {
+    z.bv[id] = s.q[0];
+#pragma unroll
+    for (int k = 1; k < 4; ++k) z.bv[id + k * sz] = s.q[k] * rho_inv;
+    z.bv[id + 4 * sz] = s.pres;
+    z.bv[id + 5 * sz] = s.T;
+  } else if (me.j == 2) {
+    for (int k = NS; k < n_scalar; ++k) z.sv[id + k * sz] = z.cv[id + (5 + k) * sz] * rho_inv;
+  }
+}
+
+// Forward and backward rate of progress of reaction r at the group's state.
+template <int NS>
+__device__ __forceinline__ void group_rate(const GroupTables<NS> &tb, const GroupMem<NS> &S, int r, double t,
+                                           double lnT, double iT, double temp_t, double itemp_t, double &q1,
+                                           double &q2) {
+  const int type = tb.type[r];
+  const uint2 mol = tb.mol[r];
+  double gf = 0, af = 1, ab = 1;
+#pragma unroll
+  for (int k = 0; k < kMaxMol; ++k) {
+    const int i = mol.x >> 8 * k & 255u, j = mol.y >> 8 * k & 255u;
+    gf += S.g[i];
+    af *= S.act[i];
+    ab *= S.act[j];
+  }
+  const double ex = fma(tb.b[r], lnT, -tb.Ea[r] * iT);
+  double kf = tb.A[r] * exp(type > 4 ? ex : ex - gf);  // with exp(-gf) in it, except for the fall-off types
+  if (type == 3) kf = fma(tb.A2[r], exp(fma(tb.b2[r], lnT, -tb.Ea2[r] * iT) - gf), kf);
+  if (type > 3) {
+    double cc = 0;
+#pragma unroll
+    for (int l = 0; l < NS; ++l) cc = fma(S.c[l], tb.tb[r][l], cc);
+    if (type == 4) {
       kf *= cc;
-    } else if (type > 4) {
-      const double kf_low = kn.A2[r] * exp(kn.b2[r] * lnT - kn.Ea2[r] * iT);
+    } else {
+      const double kf_low = tb.A2[r] * exp(fma(tb.b2[r], lnT, -tb.Ea2[r] * iT));
       const double kf_high = kf;
       if (kf_high < 1e-25 && kf_low < 1e-25) {
         kf = 0;
       } else {
-        const double pr = kf_low * cc / kf_high;
-        double F = 1.0;
+        const double pr = kf_low * cc * (1.0 / kf_high);
+        double F;  // ln of the broadening factor
         if (type > 5) {
-          double f_cent = (1 - kn.troe_alpha[r]) * exp(-t / kn.troe_t3[r]) + kn.troe_alpha[r] * exp(-t / kn.troe_t1[r]);
-          if (type == 7) f_cent += exp(-kn.troe_t2[r] * iT);
-          const double logFc = log10(f_cent);
-          const double cq = -0.4 - 0.67 * logFc;
-          const double n = 0.75 - 1.27 * logFc;
-          const double logPr = log10(pr);
-          const double tempo = (logPr + cq) / (n - 0.14 * (logPr + cq));
-          F = exp10(logFc / (1.0 + tempo * tempo));
+          const double al = tb.troe_alpha[r];
+          double f_cent = fma(1 - al, exp(-t * tb.troe_it3[r]), al * exp(-t * tb.troe_it1[r]));
+          if (type == 7) f_cent += exp(-tb.troe_t2[r] * iT);
+          // natural logarithms and one exponential for the broadening factor and exp(-gf)
+          constexpr double per_ln10 = 0.43429448190325182765;
+          const double lnFc = log(f_cent), logFc = lnFc * per_ln10;
+          const double x = fma(log(pr), per_ln10, fma(-0.67, logFc, -0.4));
+          const double tempo = x * rcp_nr(fma(-0.14, x, fma(-1.27, logFc, 0.75)));
+          F = lnFc * rcp_nr(fma(tempo, tempo, 1.0));
+        } else {
+          F = 0;
         }
-        kf = kf_high * pr / (1.0 + pr) * F;
-      }
-    }
-    double kb = 0;
-    if (type != 0) {
-      double d_gibbs = 0;
-#pragma unroll
-      for (int l = 0; l < NS; ++l)
-        if (inv >> l & 1u) d_gibbs += g[l] * (kn.stb[r][l] - kn.stf[r][l]);
-      const int o = kn.order[r];
-      double pw = 1.0;
-      for (int k = 0; k < (o < 0 ? -o : o); ++k) pw *= temp_t;
-      const double kc = (o < 0 ? 1.0 / pw : pw) * exp(-d_gibbs);
-      kb = kf / kc;
-    }
-    double a = kf, bb = kb;
-#pragma unroll
-    for (int l = 0; l < NS; ++l)
-      if (inv >> l & 1u) {
-        a *= ipow(c[l], kn.stf[r][l]);
-        bb *= ipow(c[l], kn.stb[r][l]);
-      }
-    const double q1 = a, q2 = type != 0 ? bb : 0.0;
-#pragma unroll
-    for (int l = 0; l < NS; ++l)
-      if (inv >> l & 1u) {
-        const double f = kn.stf[r][l], bq = kn.stb[r][l];
-        creation[l] += q2 * f + q1 * bq;
-        omega_d[l] += q1 * f + q2 * bq;
-      }
-    if (method == 1) {
-      // the matrix is in shared memory: its runtime row/column indices are free
-      const int ni = kn.n_inv[r];
-      for (int qa = 0; qa < ni; ++qa) {
-        const double net = kn.inv_b[r][qa] - kn.inv_f[r][qa];
-        if (net == 0) continue;
-        const int m = kn.inv_sp[r][qa];
-        for (int qb = 0; qb < ni; ++qb)
-          L(m * NS + kn.inv_sp[r][qb]) += net * (kn.inv_f[r][qb] * q1 - kn.inv_b[r][qb] * q2);
+        kf = kf_high * pr * rcp_nr(1.0 + pr) * exp(F - gf);
       }
     }
   }
-  double omega[NS];
+  q1 = kf * af;
+  // kb = kf / Kc carries (p_atm / R_u T)^-order
+  q2 = type != 0 ? kf * ab : 0.0;
+  const int o = tb.order[r];
+  for (int k = 0; k < (o < 0 ? -o : o); ++k) q2 *= o < 0 ? temp_t : itemp_t;
+}
+
+// A row is swapped in as pivot only if its entry is more than this many times
+// the diagonal's (threshold pivoting).
+constexpr double kPivotThreshold = 4.0;
+
+// Solves the group's system by Gauss-Jordan elimination with threshold
+// pivoting: a[k][m] is row m of the lane's column k GL + j, x the right-hand
+// side, the same in all lanes; y receives the lane's unknowns.  The owner of
+// a column picks its pivot and passes its multipliers on.  Rows are swapped,
+// by the whole warp, only if some group's pivot is off the diagonal.
+template <int NS, int GL>
+__device__ __forceinline__ void group_solve(double (&a)[NS / GL][NS], double (&x)[NS], const Lane<NS, GL> &me,
+                                            double (&y)[NS / GL]) {
+  constexpr int SPL = NS / GL;
+  double inv[SPL];
 #pragma unroll
-  for (int l = 0; l < NS; ++l) {
-    const double w = 1e+3 / th->imw[l];
-    creation[l] *= w;
-    omega_d[l] *= w;
-    omega[l] = creation[l] - omega_d[l];
+  for (int i = 0; i < NS; ++i) {
+    const int k = i / GL, src = me.base + i % GL;
+    int p = i;
+    double best = kPivotThreshold * fabs(a[k][i]);
+#pragma unroll
+    for (int m = i + 1; m < NS; ++m)
+      if (fabs(a[k][m]) > best) {
+        best = fabs(a[k][m]);
+        p = m;
+      }
+    p = __shfl_sync(0xffffffffu, p, src);
+    if (__any_sync(0xffffffffu, p != i)) {
+#pragma unroll
+      for (int m = i + 1; m < NS; ++m) {
+        const bool sw = p == m;
+#pragma unroll
+        for (int c = k; c < SPL; ++c) {
+          const double u = a[c][i], v = a[c][m];
+          a[c][i] = sw ? v : u;
+          a[c][m] = sw ? u : v;
+        }
+        const double u = x[i], v = x[m];
+        x[i] = sw ? v : u;
+        x[m] = sw ? u : v;
+      }
+    }
+    const double r = rcp_nr(a[k][i]);
+    if (me.j == i % GL) inv[k] = r;
+#pragma unroll
+    for (int m = 0; m < NS; ++m) {
+      if (m == i) continue;
+      const double f = __shfl_sync(0xffffffffu, a[k][m] * r, src);
+      // the columns up to i are done: their entries are no longer read
+#pragma unroll
+      for (int c = (i % GL == GL - 1 ? k + 1 : k); c < SPL; ++c) a[c][m] = fma(-f, a[c][i], a[c][m]);
+      x[m] = fma(-f, x[i], x[m]);
+    }
   }
 #pragma unroll
-  for (int l = 0; l < NS; ++l) c[l] *= 1e+3 / th->imw[l];
+  for (int k = 0; k < SPL; ++k) {
+    double v = x[k * GL];
+#pragma unroll
+    for (int j = 1; j < GL; ++j)
+      if (me.j == j) v = x[k * GL + j];
+    y[k] = v * inv[k];
+  }
+}
+
+// One substep of wu_zeroDReaction (methods 0 and 1) of a warp's groups, all
+// lanes of the warp together; `on`: the lane's group has a node and a step to
+// take (the others compute along and keep their state).
+template <int NS, int GL>
+__device__ __forceinline__ bool group_substep(const Zone &z, const GroupTables<NS> &tb, GroupMem<NS> &S,
+                                              const Lane<NS, GL> &me, int n_reac, int method, double dt, bool on,
+                                              GroupState<NS / GL> &s) {
+  constexpr int SPL = NS / GL;
+  const double t = s.T, lnT = log(t), iT = rcp_nr(t);
+#pragma unroll
+  for (int k = 0; k < SPL; ++k) {
+    const int i = k * GL + me.j;
+    const double c = s.rY[k] * tb.imw3[i];
+    const double g = gibbs_one(tb.low[i], tb.high[i], me.t_low[k], me.t_mid[k], me.t_high[k], t, lnT, iT);
+    if (me.own) {
+      S.c[i] = c;
+      S.g[i] = g;
+      S.act[i] = c * exp(g);
+    }
+  }
+  __syncwarp();
+  constexpr double temp_p = 101325.0 / kRu * 1e-3;  // mol K / cm^3
+  const double temp_t = temp_p * iT, itemp_t = t * (1.0 / temp_p);
+  if (me.own)
+    for (int k = me.j; k < n_reac; k += GL) {
+      const int r = tb.deal[k];
+      double q1, q2;
+      group_rate<NS>(tb, S, r, t, lnT, iT, temp_t, itemp_t, q1, q2);
+      S.q1[r] = q1;
+      S.q2[r] = q2;
+    }
+  __syncwarp();
+  // the lane's species: creation, destruction and its columns of the matrix
+  double a[SPL][NS], y[SPL], tsl = 1e6;
+#pragma unroll
+  for (int k = 0; k < SPL; ++k) {
+    // minus the column's scale: dt 1e3 W_n / rhoY_n
+    const double w = 1e+3 * me.mw[k], sn = s.rY[k] > 1e-25 ? -dt * w * rcp_nr(s.rY[k]) : 0.0;
+    double make = 0, use = 0;
+#pragma unroll
+    for (int m = 0; m < NS; ++m) a[k][m] = m == k * GL + me.j ? 1.0 : 0.0;
+    for (int e = me.ent[k]; e < me.ent_end[k]; ++e) {
+      const int r = tb.ent_r[e];
+      const double f = tb.ent_f[e], b = tb.ent_b[e], q1 = S.q1[r], q2 = S.q2[r];
+      make = fma(q2, f, fma(q1, b, make));
+      use = fma(q1, f, fma(q2, b, use));
+      if (method == 1) {
+        const double d = sn * fma(f, q1, -b * q2);
+#pragma unroll
+        for (int m = 0; m < NS; ++m) a[k][m] = fma(tb.net[r][m], d, a[k][m]);
+      }
+    }
+    y[k] = 1e+3 * (make - use);
+    use *= w;
+    if (s.rY[k] > 1e-25 && fabs(use) > 1e-25) tsl = fmin(tsl, fabs(s.rY[k] * rcp_nr(use)));
+  }
   if (method == 1) {
-    // (I - dt J): J_mn / rhoY_n * 1e3 / imw_m, with the 2 NS divisions hoisted
-    double rc[NS], wm[NS];
+    if (me.own) {
 #pragma unroll
-    for (int n = 0; n < NS; ++n) {
-      rc[n] = c[n] > 1e-25 ? 1.0 / c[n] : 0.0;
-      wm[n] = 1e+3 / th->imw[n];
+      for (int k = 0; k < SPL; ++k) S.w[k * GL + me.j] = y[k];
     }
+    __syncwarp();
+    double x[NS];
 #pragma unroll
-    for (int m = 0; m < NS; ++m)
-#pragma unroll
-      for (int n = 0; n < NS; ++n) L(m * NS + n) = (m == n ? 1 : 0) - dt * (L(m * NS + n) * rc[n] * wm[m]);
-#pragma unroll
-    for (int l = 0; l < NS; ++l) R(l) = omega[l];
-    lu_solve_ns<NS>(L, R, omega);
+    for (int m = 0; m < NS; ++m) x[m] = S.w[m];
+    group_solve<NS, GL>(a, x, me, y);
   }
+  double q[5], cnY[SPL];
 #pragma unroll
-  for (int l = 0; l < 5; ++l) s.q[l] += s.cn[l] * dt * s.iJac;
-  double time_scale = 1e6;
+  for (int k = 0; k < SPL; ++k) cnY[k] = 0;
 #pragma unroll
-  for (int l = 0; l < NS; ++l) {
-    if (s.rY[l] > 1e-25 && abs(omega_d[l]) > 1e-25) time_scale = min(time_scale, abs(s.rY[l] / omega_d[l]));
-    s.rY[l] += (omega[l] + s.cnY[l] * s.iJac) * dt;
+  for (int k = 0; k < 5; ++k) q[k] = s.q[k];
+  if (z.Cn) {
+    const int64_t szq = z.d.plane(0);
+#pragma unroll
+    for (int k = 0; k < 5; ++k) q[k] = fma(z.Cn[s.iq + k * szq], dt * s.iJac, q[k]);
+#pragma unroll
+    for (int k = 0; k < SPL; ++k) cnY[k] = z.Cn[s.iq + (5 + me.sp[k]) * szq] * s.iJac;
   }
-  s.ts = time_scale;
-  const double rho = s.q[0];
-  const double rho_inv = 1.0 / rho;
-  const double u = s.q[1] * rho_inv, v = s.q[2] * rho_inv, w = s.q[3] * rho_inv;
-  double sum = 0;
+  double nY[SPL], part = 0;
 #pragma unroll
-  for (int l = 0; l < NS; ++l) {
-    if (s.rY[l] < 0) s.rY[l] = 0;
-    else sum += s.rY[l];
+  for (int k = 0; k < SPL; ++k) {
+    nY[k] = fma(fma(y[k], me.mw[k], cnY[k]), dt, s.rY[k]);
+    if (nY[k] < 0) nY[k] = 0;
+    part = __dadd_rn(part, nY[k]);
   }
-  sum = 1.0 / sum;
-  const double ratio = rho * sum;
+  const double sum = rcp_nr(me.sum(part)), ts = me.min(tsl);
+  const double rho = q[0], rho_inv = rcp_nr(rho), ratio = rho * sum;
+  const double u = q[1] * rho_inv, v = q[2] * rho_inv, w = q[3] * rho_inv;
+  double Y[SPL];
+  part = 0;
 #pragma unroll
-  for (int l = 0; l < NS; ++l) {
-    yk[l] = s.rY[l] * sum;
-    s.rY[l] *= ratio;
+  for (int k = 0; k < SPL; ++k) {
+    Y[k] = nY[k] * sum;
+    nY[k] *= ratio;
+    part = fma(Y[k], me.R[k], part);
   }
-  return temperature_newton_ns<NS>(th, yk, s.q[4], rho, u * u + v * v + w * w, s.T, pres);
+  // T by Newton's iteration from the energy (temperature_newton)
+  const double gas_const = me.sum(part);
+  const double e = fma(-0.5, fma(u, u, fma(v, v, w * w)), q[4] * rho_inv);
+  double T = t, err = 1;
+  for (int iter = 0; iter < 1000; ++iter) {
+    const bool go = on && err > 1e-5;
+    if (!__any_sync(0xffffffffu, go)) break;
+    double h = 0, cp = 0;
+#pragma unroll
+    for (int k = 0; k < SPL; ++k) {
+      const int i = k * GL + me.j;
+      const double tt = fmin(fmax(T, me.t_low[k]), me.t_high[k]);
+      const double *c = T < me.t_mid[k] ? tb.low[i] : tb.high[i];
+      const double p0 = fma(tt, fma(tt, fma(tt, fma(tt, c[4], c[3]), c[2]), c[1]), c[0]);
+      const double p1 =
+          fma(tt, fma(tt, fma(tt, fma(tt, 0.2 * c[4], 0.25 * c[3]), (1.0 / 3) * c[2]), 0.5 * c[1]), c[0]);
+      const double ry = me.R[k] * Y[k];
+      cp = fma(ry, p0, cp);
+      h = fma(ry, fma(p0, T - tt, fma(tt, p1, c[5])), h);
+    }
+    h = me.sum(h);
+    cp = me.sum(cp);
+    if (go) {
+      const double t1 = fma(e - fma(-gas_const, T, h), rcp_nr(cp - gas_const), T);
+      err = fabs(fma(-t1, rcp_nr(T), 1.0));
+      T = t1;
+    }
+  }
+  if (on) {
+#pragma unroll
+    for (int k = 0; k < 5; ++k) s.q[k] = q[k];
+#pragma unroll
+    for (int k = 0; k < SPL; ++k) {
+      s.rY[k] = nY[k];
+      s.Y[k] = Y[k];
+    }
+    s.ts = ts;
+    s.T = T;
+    s.pres = rho * T * gas_const;
+  }
+  return !on || err <= 1e-5;
 }
 
 }  // namespace cfk

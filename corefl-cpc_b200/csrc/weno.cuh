@@ -6,18 +6,6 @@
 
 namespace cfk {
 
-// 1/x for x whose reciprocal is a normal number: the hardware's 20-bit
-// approximation (PTX rcp.approx.ftz.f64) and one third-order Householder step
-// y (1 + e + e^2), e = 1 - x y, whose remainder e^3 is below 2^-60; the result
-// is within 2 ulp.  Three FMAs, against a division sequence with its range
-// checks.  x = 0 and x = inf give NaN.
-__device__ __forceinline__ double rcp_nr(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-
 // Dot products with a fixed order of FMAs.  Where the compiler chooses which
 // product of a sum to fuse, the choice can differ between the instantiations
 // of a kernel; the tile shapes of a sweep give bit-identical fluxes.

@@ -128,3 +128,40 @@ def test_ignition_of_the_reference_reactor_case():
     assert Ts[-1] == pytest.approx(golden["T"][-1], rel=1e-5)
     t_ign = np.interp(1500.0, Ts, ts)
     assert t_ign == pytest.approx(8.88e-4, rel=0.01)
+
+
+@pytest.mark.parametrize("n", [1, 9, 10, 11, 39, 41, 121])
+@pytest.mark.parametrize("long_side", [False, True])
+def test_reaction_step_at_group_edges(n, long_side):
+    """Node counts around the nodes of a warp (10) and of a CTA (40), both
+    schedules, uneven substep counts.  long_side: a reaction with four
+    molecules on a side, which the lane-group kernels' species lists do not
+    hold, takes the runtime-count kernels."""
+    import dataclasses
+
+    mech = mechanism.load("li2004")
+    if long_side:
+        r = next(k for k in range(mech.n_reac) if mech.stoi_f[k].max() == 2)
+        f, b = np.array(mech.stoi_f), np.array(mech.stoi_b)
+        f[r] *= 2
+        b[r] *= 2
+        mech = dataclasses.replace(mech, stoi_f=f, stoi_b=b)
+    case = cases.reactor_batch(mech, n, seed=n)
+    oz, gz = _pair(case)
+    nsub = _nsub_tensor(gz)
+    oz["reaction_timeScale"][:] = 1e-7 / (0.5 + 3 + np.arange(n) % 23)
+    for s in range(3):
+        ns_o = None
+        for schedule in (0, 1):
+            gz.load_from(oz, keys=("cv", "bv", "sv", "reaction_timeScale"))
+            gz.ctx.wu_reaction_step(1e-7, schedule=schedule, nsub_ptr=nsub.data_ptr())
+            gz.ctx.sync()
+            out = {k: gz.get(k).copy() for k in ("cv", "bv", "sv", "reaction_timeScale")}
+            if ns_o is None:
+                first, ns_o = out, nsub.cpu().numpy().copy()
+            else:
+                assert all(np.array_equal(out[k], first[k]) for k in out)
+        ns_r = oz.reaction_step(1e-7, want_nsub=True)
+        assert np.array_equal(ns_o, ns_r)
+        assert rel_err(out["cv"], oz["cv"]) <= 1e-12
+        assert rel_err(out["sv"], oz["sv"], momentum=()) <= 1e-11  # the smallest species, against its own maximum
