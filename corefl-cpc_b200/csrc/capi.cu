@@ -3,6 +3,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -471,6 +472,7 @@ int cfk_set_mechanism(cfk_ctx *c, const cfk_mechanism *m) {
     for (int q = 0; q < 7; ++q) { th.low[l][q] = m->low[l][q]; th.high[l][q] = m->high[l][q]; }
     th.geometry[l] = m->geometry[l];
     th.LJ_potent_inv[l] = m->LJ_potent_inv[l];
+    th.LJ_pow[l] = std::pow(m->LJ_potent_inv[l], -0.145);
     th.vis_coeff[l] = m->vis_coeff[l];
     th.ZRotF298[l] = m->ZRotF298[l];
     for (int n = 0; n < ns; ++n) {
@@ -478,6 +480,8 @@ int cfk_set_mechanism(cfk_ctx *c, const cfk_mechanism *m) {
       th.sqrt_WiDivWjPl1Mul8[l][n] = m->sqrt_WiDivWjPl1Mul8[l][n];
       th.binary_diffusivity_coeff[l][n] = m->binary_diffusivity_coeff[l][n];
       th.kb_over_eps_jk[l][n] = m->kb_over_eps_jk[l][n];
+      th.kb_pow[l][n] = std::pow(m->kb_over_eps_jk[l][n], -0.15504);
+      th.inv_bdc[l][n] = 1.0 / m->binary_diffusivity_coeff[l][n];
     }
   }
   Kinetics &kn = h.kn;

@@ -28,17 +28,6 @@
 
 namespace cfk {
 
-// h and cp (J/kg, J/kg/K) of species i, extrapolated linearly outside its
-// range: the polynomials are taken at the clamped temperature, so inside the
-// range the extrapolation adds zero, and no branch is left.
-__device__ __forceinline__ void enthalpy_cp_one(const Thermo *th, int i, double t, double &h, double &cp) {
-  const double tt = fmin(fmax(t, th->t_low[i]), th->t_high[i]);
-  const double *c = t < th->t_mid[i] ? th->low[i] : th->high[i];
-  cp = th->gas_const[i] * fma(tt, fma(tt, fma(tt, fma(tt, c[4], c[3]), c[2]), c[1]), c[0]);
-  const double p = fma(tt, fma(tt, fma(tt, fma(tt, 0.2 * c[4], 0.25 * c[3]), (1.0 / 3) * c[2]), 0.5 * c[1]), c[0]);
-  h = fma(th->gas_const[i], fma(tt, p, c[5]), cp * (t - tt));
-}
-
 template <int NS>
 __device__ __forceinline__ void enthalpy_cp_ns(const Thermo *th, double t, double *h, double *cp) {
 #pragma unroll
