@@ -1,6 +1,8 @@
 // Node-local kernels of the stage: SSP-RK3 update, property update, cv from
 // bv, local CFL step with its grid minimum, boundary faces and the 2-D
 // k-ghost copy.  All are HBM-bound; each touches a node's planes once.
+#include <algorithm>
+
 #include "cfk_common.cuh"
 #include "thermo.cuh"
 #include "cv_point.cuh"
@@ -241,6 +243,47 @@ __global__ void update_physical_properties_kernel(Zone z, Param p, const Thermo 
   }
 }
 
+// The shell of a 3-D block (see above) by its own index: of each axis the
+// ghost layers and the outermost node on either side, first whole k planes,
+// then the j rows and last the i ends of what is left.  Launched over the
+// padded block, a warp in an interior row would compute for its few shell
+// lanes what it computes for 32.
+__device__ __forceinline__ int shell_coord(int o, int m, int g) {
+  return m < 2 || o <= g ? o - g : m - 1 + (o - (g + 1));  // o counts the axis' shell nodes upwards
+}
+
+template <bool MIX>
+__global__ void __launch_bounds__(128) shell_properties_kernel(Zone z, Param p, const Thermo *th, long long total) {
+  const Dims d = z.d;
+  const int g = d.ngg;
+  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
+  const int sx = d.sx(g), sy = d.sy(g);
+  const int nx = max(d.mx - 2, 0), ny = max(d.my - 2, 0), nz = max(d.mz - 2, 0);  // inner nodes
+  const int ox = sx - nx, oy = sy - ny, oz = d.mz + 2 * g - nz;                   // shell nodes of an axis
+  int i, j, k;
+  const long long nk = (long long)oz * sx * sy, nj = (long long)nz * oy * sx;
+  if (t < nk) {
+    k = shell_coord((int)(t / (sx * sy)), d.mz, g);
+    const int r = (int)(t % (sx * sy));
+    j = r / sx - g;
+    i = r % sx - g;
+  } else if (t < nk + nj) {
+    t -= nk;
+    k = (int)(t / (oy * sx)) + 1;
+    const int r = (int)(t % (oy * sx));
+    j = shell_coord(r / sx, d.my, g);
+    i = r % sx - g;
+  } else {
+    t -= nk + nj;
+    const long long row = t / ox;
+    k = (int)(row / ny) + 1;
+    j = (int)(row % ny) + 1;
+    i = shell_coord((int)(t - row * ox), d.mx, g);
+  }
+  properties_point<MIX>(z, p, th, d.idx(g, i, j, k));
+}
+
 // ---------------------------------------------------------------------------
 // local_time_step (reference src/TimeAdvanceFunc.cuh:28-115) fused with the
 // grid minimum of global_time_step (reference src/TimeAdvanceFunc.cu:102-152):
@@ -322,6 +365,8 @@ __global__ void reset_dt_kernel(unsigned long long *bits) { *bits = (unsigned lo
 struct FaceGeom {
   int face, direction;
   int lo[3], n[3];  // range start and extent per axis
+  int parts;        // threads sharing a face node (face_work)
+  int pair;         // 1: the launch also does the opposite face
 };
 
 __device__ __forceinline__ void face_node(const FaceGeom &fg, int t, int &i, int &j, int &k) {
@@ -330,24 +375,38 @@ __device__ __forceinline__ void face_node(const FaceGeom &fg, int t, int &i, int
   i = fg.lo[0] + a; j = fg.lo[1] + b; k = fg.lo[2] + c;
 }
 
-// Work split of a boundary-face kernel.  On i faces the ghost layers of a
-// face node are consecutive in memory, so ngg + 1 threads share a node: part
-// 0 does the face node's own work, part gg fills ghost layer gg (the ghost
-// fills read interior nodes only, never the face node, so the parts are
-// independent); the lanes of a warp then cover whole runs of ghost cells
-// instead of one cell per row.  On j and k faces one thread does the node and
-// all its ghost layers, the lanes running along i.
-__device__ __forceinline__ bool face_work(const FaceGeom &fg, int g, int &i, int &j, int &k, int &gg_lo,
-                                          int &gg_hi, bool &face_part) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int parts = fg.face == 0 ? g + 1 : 1;
-  const int node = t / parts, part = t - node * parts;
-  if (node >= fg.n[0] * fg.n[1] * fg.n[2]) return false;
+// Work split of a boundary-face kernel.  ngg + 1 threads share a face node:
+// part 0 does the face node's own work, part gg fills ghost layer gg (the ghost
+// fills read interior nodes only, never a face node, so the parts are
+// independent), and the two faces of an axis are one launch where both carry
+// the same condition.  Where the block is too thin for that (an inner node of
+// one face is the other face's node: make_face) one thread does a node and all
+// its layers, and each face is its own launch.  On i faces the ghost layers of
+// a face node are consecutive in memory and the parts run along the lanes; on j
+// and k faces the lanes run along i.  A face is a few thousand nodes: with one
+// thread a node its four layers were a serial chain (periodic j/k face of a 97
+// x 49 x 33 mixture block 61 us).
+__device__ __forceinline__ bool face_work(const FaceGeom &fg, const Dims &d, int &i, int &j, int &k, int &gg_lo,
+                                          int &gg_hi, bool &face_part, int &dir) {
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nodes = fg.n[0] * fg.n[1] * fg.n[2], work = nodes * fg.parts;
+  dir = fg.direction;
+  int shift = 0;
+  if (fg.pair && t >= work) {
+    t -= work;
+    dir = -dir;
+    shift = fg.direction < 0 ? d.ext(fg.face) - 1 : 1 - d.ext(fg.face);
+  }
+  if (t >= work) return false;
+  const int node = fg.face == 0 ? t / fg.parts : t % nodes, part = fg.face == 0 ? t % fg.parts : t / nodes;
   face_node(fg, node, i, j, k);
-  face_part = fg.face != 0 || part == 0;
-  gg_lo = fg.face == 0 ? part : 1;
-  gg_hi = fg.face == 0 ? part : g;
-  if (fg.face == 0 && part == 0) { gg_lo = 1; gg_hi = 0; }
+  if (fg.face == 0) i += shift;
+  else if (fg.face == 1) j += shift;
+  else k += shift;
+  face_part = part == 0;
+  gg_lo = fg.parts == 1 ? 1 : part;
+  gg_hi = fg.parts == 1 ? d.ngg : part;
+  if (fg.parts > 1 && part == 0) { gg_lo = 1; gg_hi = 0; }
   return true;
 }
 
@@ -364,11 +423,11 @@ template <bool MIX>
 __global__ void bc_outflow_kernel(Zone z, Param p, const Thermo *th, FaceGeom fg, cfk_outflow of) {
   const Dims d = z.d;
   const int g = d.ngg;
-  int i, j, k, gg_lo, gg_hi;
+  int i, j, k, gg_lo, gg_hi, dir;
   bool face_part;
-  if (!face_work(fg, g, i, j, k, gg_lo, gg_hi, face_part)) return;
+  if (!face_work(fg, d, i, j, k, gg_lo, gg_hi, face_part, dir)) return;
   const int64_t sz = d.plane(g), id = d.idx(g, i, j, k);
-  const int64_t s = d.stride(g, fg.face) * fg.direction;
+  const int64_t s = d.stride(g, fg.face) * dir;
   if (!of.back_pressure_on) {
     for (int gg = gg_lo; gg <= gg_hi; ++gg) {
       const int64_t gi = id + gg * s;
@@ -381,7 +440,7 @@ __global__ void bc_outflow_kernel(Zone z, Param p, const Thermo *th, FaceGeom fg
   if (gg_lo > gg_hi) return;
   const int mf = 3 * fg.face;
   double nx = z.metric[id + mf * sz], ny = z.metric[id + (mf + 1) * sz], nz = z.metric[id + (mf + 2) * sz];
-  const double grad_n_inv = fg.direction / sqrt(nx * nx + ny * ny + nz * nz);
+  const double grad_n_inv = dir / sqrt(nx * nx + ny * ny + nz * nz);
   nx *= grad_n_inv;
   ny *= grad_n_inv;
   nz *= grad_n_inv;
@@ -463,11 +522,11 @@ template <bool MIX>
 __global__ void bc_symmetry_kernel(Zone z, Param p, const Thermo *th, FaceGeom fg) {
   const Dims d = z.d;
   const int g = d.ngg;
-  int i, j, k, gg_lo, gg_hi;
+  int i, j, k, gg_lo, gg_hi, dir;
   bool face_part;
-  if (!face_work(fg, g, i, j, k, gg_lo, gg_hi, face_part)) return;
+  if (!face_work(fg, d, i, j, k, gg_lo, gg_hi, face_part, dir)) return;
   const int64_t sz = d.plane(g), id = d.idx(g, i, j, k);
-  const int64_t s = d.stride(g, fg.face) * fg.direction;
+  const int64_t s = d.stride(g, fg.face) * dir;
   const int64_t in = id - s;
   const int mf = 3 * fg.face;
   double k_x = z.metric[id + mf * sz], k_y = z.metric[id + (mf + 1) * sz], k_z = z.metric[id + (mf + 2) * sz];
@@ -503,15 +562,15 @@ template <bool MIX>
 __global__ void bc_periodic_kernel(Zone z, Param p, const Thermo *th, FaceGeom fg) {
   const Dims d = z.d;
   const int g = d.ngg;
-  int i, j, k, gg_lo, gg_hi;
+  int i, j, k, gg_lo, gg_hi, dir;
   bool face_part;
-  if (!face_work(fg, g, i, j, k, gg_lo, gg_hi, face_part)) return;
+  if (!face_work(fg, d, i, j, k, gg_lo, gg_hi, face_part, dir)) return;
   const int64_t sz = d.plane(g), id = d.idx(g, i, j, k);
   const int64_t sd = d.stride(g, fg.face);
-  const int64_t s = sd * fg.direction;
+  const int64_t s = sd * dir;
   const int mface = d.ext(fg.face);
-  const int64_t io = id + (int64_t)(fg.direction < 0 ? (mface - 1) : -(mface - 1)) * sd;
-  if (face_part) {
+  const int64_t io = id + (int64_t)(dir < 0 ? (mface - 1) : -(mface - 1)) * sd;
+  if (face_part && !(fg.pair && dir != fg.direction)) {  // of a pair, one side writes both face nodes
     for (int l = 0; l < 6; ++l) {
       const double ave = 0.5 * (z.bv[id + l * sz] + z.bv[io + l * sz]);
       z.bv[id + l * sz] = ave;
@@ -523,6 +582,7 @@ __global__ void bc_periodic_kernel(Zone z, Param p, const Thermo *th, FaceGeom f
       z.sv[io + l * sz] = ave;
     }
     cv_from_bv_point<MIX>(z, p, th, id);
+    if (fg.pair) cv_from_bv_point<MIX>(z, p, th, io);
   }
   for (int gg = gg_lo; gg <= gg_hi; ++gg) {
     const int64_t gi = id + gg * s, ii = io + gg * s;
@@ -665,11 +725,11 @@ template <bool MIX>
 __global__ void bc_wall_kernel(Zone z, Param p, const Thermo *th, FaceGeom fg, cfk_wall wall) {
   const Dims d = z.d;
   const int g = d.ngg;
-  int i, j, k, gg_lo, gg_hi;
+  int i, j, k, gg_lo, gg_hi, dir;
   bool face_part;
-  if (!face_work(fg, g, i, j, k, gg_lo, gg_hi, face_part)) return;
+  if (!face_work(fg, d, i, j, k, gg_lo, gg_hi, face_part, dir)) return;
   const int64_t sz = d.plane(g), id = d.idx(g, i, j, k);
-  const int64_t s = d.stride(g, fg.face) * fg.direction;
+  const int64_t s = d.stride(g, fg.face) * dir;
   const bool isothermal = wall.thermal_type == 0;
   const bool catalytic = MIX && wall.catalytic_type == 1;
   if (face_part) {
@@ -775,19 +835,25 @@ __global__ void inner_face_kernel(Zone z, Zone tz, Param p, const Thermo *th, cf
 }
 
 // eliminate_k_gradient (reference src/FieldOperation.cu:47-72)
+// One thread a copied node: grid.z runs over the 2 ngg ghost planes.
 __global__ void eliminate_k_gradient_kernel(Zone z, Param p) {
   const Dims d = z.d;
   const int g = d.ngg;
   const int i = blockIdx.x * blockDim.x + threadIdx.x - g;
-  const int j = blockIdx.y - g;
+  const int j = blockIdx.y - g, k = (int)blockIdx.z < g ? (int)blockIdx.z - g : (int)blockIdx.z - g + 1;
   if (i >= d.mx + g) return;
-  const int64_t sz = d.plane(g), i0 = d.idx(g, i, j, 0);
-  for (int k = 1; k <= g; ++k) {
-    const int64_t ip = d.idx(g, i, j, k), im = d.idx(g, i, j, -k);
-    for (int l = 0; l < 6; ++l) { z.bv[ip + l * sz] = z.bv[i0 + l * sz]; z.bv[im + l * sz] = z.bv[i0 + l * sz]; }
-    for (int l = 0; l < p.n_scalar; ++l) { z.sv[ip + l * sz] = z.sv[i0 + l * sz]; z.sv[im + l * sz] = z.sv[i0 + l * sz]; }
-    for (int l = 0; l < p.n_var; ++l) { z.cv[ip + l * sz] = z.cv[i0 + l * sz]; z.cv[im + l * sz] = z.cv[i0 + l * sz]; }
-  }
+  const int64_t sz = d.plane(g), i0 = d.idx(g, i, j, 0), ik = d.idx(g, i, j, k);
+#pragma unroll
+  for (int l = 0; l < 6; ++l) z.bv[ik + l * sz] = z.bv[i0 + l * sz];
+  for (int l = 0; l < p.n_scalar; ++l) z.sv[ik + l * sz] = z.sv[i0 + l * sz];
+#pragma unroll 5
+  for (int l = 0; l < p.n_var; ++l) z.cv[ik + l * sz] = z.cv[i0 + l * sz];
+}
+
+static void launch_eliminate_k(const Zone &z, const Param &p, cudaStream_t st) {
+  const int g = z.d.ngg;
+  if (g < 1) return;
+  eliminate_k_gradient_kernel<<<dim3((z.d.mx + 2 * g + 127) / 128, z.d.my + 2 * g, 2 * g), 128, 0, st>>>(z, p);
 }
 
 // ---------------------------------------------------------------------------
@@ -831,6 +897,15 @@ cudaError_t launch_cv_from_bv(const Zone &z, const Param &p, const Thermo *th, c
 cudaError_t launch_update_properties(const Zone &z, const Param &p, const Thermo *th, cudaStream_t st, bool shell,
                                      bool planar) {
   dim3 grid = padded_grid(z.d, 128);
+  if (shell && z.d.mz > 1) {
+    const Dims &d = z.d;
+    const long long inner = (long long)std::max(d.mx - 2, 0) * std::max(d.my - 2, 0) * std::max(d.mz - 2, 0);
+    const long long total = d.plane(d.ngg) - inner;
+    const unsigned blocks = (unsigned)((total + 127) / 128);
+    if (p.n_spec > 0) shell_properties_kernel<true><<<blocks, 128, 0, st>>>(z, p, th, total);
+    else shell_properties_kernel<false><<<blocks, 128, 0, st>>>(z, p, th, total);
+    return cudaGetLastError();
+  }
   planar = planar && z.d.mz == 1;
   if (planar) grid.y = 1;
   if (p.n_spec > 0) update_physical_properties_kernel<true><<<grid, 128, 0, st>>>(z, p, th, shell, planar);
@@ -870,6 +945,10 @@ static FaceGeom make_face(const Dims &d, const cfk_face &f, int viscous_order) {
     }
   }
   if (d.mz == 1) { fg.lo[2] = -g; fg.n[2] = 2 * g + 1; }
+  // the inner nodes a face's ghosts are filled from, up to ngg away, are
+  // interior ones
+  fg.parts = m[f.face] > d.ngg + 1 && f.label != 5 ? d.ngg + 1 : 1;
+  fg.pair = 0;
   return fg;
 }
 
@@ -879,11 +958,18 @@ cudaError_t launch_boundary_conditions(const Zone &z, const Param &p, const Ther
   // reference priority order: outflow, inflow, symmetry, wall, periodic
   static const int order[5] = {6, 5, 3, 2, 8};
   for (int o = 0; o < 5; ++o) {
+    bool done[6] = {};
     for (int n = 0; n < n_face; ++n) {
-      if (faces[n].label != order[o]) continue;
-      const FaceGeom fg = make_face(z.d, faces[n], p.viscous_order);
-      const bool split = order[o] != 5;  // the inflow kernel keeps a face node's line in one thread
-      const int cnt = fg.n[0] * fg.n[1] * fg.n[2] * (split && fg.face == 0 ? z.d.ngg + 1 : 1);
+      if (faces[n].label != order[o] || done[n]) continue;
+      FaceGeom fg = make_face(z.d, faces[n], p.viscous_order);
+      // the opposite face, if it is the next one of this condition, in the same launch
+      int next = n + 1;
+      while (next < n_face && faces[next].label != order[o]) ++next;
+      if (fg.parts > 1 && next < n_face && faces[next].face == fg.face && faces[next].direction == -fg.direction) {
+        fg.pair = 1;
+        done[next] = true;
+      }
+      const int cnt = fg.n[0] * fg.n[1] * fg.n[2] * fg.parts * (1 + fg.pair);
       const int blocks = (cnt + 127) / 128;
       const bool mix = p.n_spec > 0;
       if (order[o] == 6) {
@@ -912,14 +998,14 @@ cudaError_t launch_boundary_conditions(const Zone &z, const Param &p, const Ther
     }
   }
   if (z.d.mz == 1) {
-    eliminate_k_gradient_kernel<<<dim3((z.d.mx + 2 * z.d.ngg + 127) / 128, z.d.my + 2 * z.d.ngg), 128, 0, st>>>(z, p);
+    launch_eliminate_k(z, p, st);
     ++*n_launch;
   }
   return cudaGetLastError();
 }
 
 cudaError_t launch_eliminate_k_gradient(const Zone &z, const Param &p, cudaStream_t st) {
-  eliminate_k_gradient_kernel<<<dim3((z.d.mx + 2 * z.d.ngg + 127) / 128, z.d.my + 2 * z.d.ngg), 128, 0, st>>>(z, p);
+  launch_eliminate_k(z, p, st);
   return cudaGetLastError();
 }
 

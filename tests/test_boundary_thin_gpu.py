@@ -1,0 +1,72 @@
+"""Boundary faces and the properties shell of blocks around the extents at
+which a face's ghost layers stop being shared between threads and its two
+faces stop being one launch (ngg + 1 nodes), against the CPU oracle.
+
+The faces copy, average and reflect; cv is then one product and sum a value:
+1e-14 of each plane's largest value."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+import cases
+import mechanism
+import pyoracle
+from gpuzone import GpuZone, rel_err
+
+pytestmark = pytest.mark.gpu
+
+LABELS = {"periodic": [(a, d, 8) for a in range(3) for d in (-1, 1)],
+          "outflow": [(a, d, 6) for a in range(3) for d in (-1, 1)],
+          "symmetry": [(a, d, 3) for a in range(3) for d in (-1, 1)],
+          # the two faces of an axis apart in the list, or of two conditions: a launch each
+          "mixed": [(0, -1, 6), (1, -1, 6), (0, 1, 6), (1, 1, 3), (2, -1, 8), (2, 1, 8)]}
+
+
+def _corner(case, n, ny, nz):
+    """The first n x ny x nz nodes of a block, with its padded arrays' values."""
+    g = case.ngg
+
+    def cut(a):
+        a = a.reshape(a.shape[:-1] + case.shape())[..., : nz + 2 * g, : ny + 2 * g, : n + 2 * g]
+        return np.ascontiguousarray(a.reshape(a.shape[:-3] + (-1,)))
+
+    return dataclasses.replace(case, mx=n, my=ny, mz=nz, metric=cut(case.metric), jac=cut(case.jac), bv=cut(case.bv),
+                               sv=np.zeros((0, cut(case.jac).size)), x=None, xyz=None)
+
+
+@pytest.mark.parametrize("labels", list(LABELS))
+@pytest.mark.parametrize("shape", [(9, 8, 7), (5, 4, 6), (4, 6, 5), (12, 5, 4)])
+@pytest.mark.parametrize("viscous", [False, True])
+def test_boundary_conditions_of_thin_blocks(labels, shape, viscous):
+    case = _corner(cases.perturbed(cases.sine_wave(n=13, ny=9, nz=9, scheme=52, viscous=viscous, amp=0.02), seed=1,
+                                   amp=0.05), *shape)
+    if labels == "symmetry" and min(shape) < 5:
+        pytest.skip("a reflected node of one symmetry face would be the other's")
+    case.faces = LABELS[labels]
+    oz = pyoracle.OracleZone(case)
+    oz.call("orc_compute_cv_from_bv")
+    gz = GpuZone(case)
+    gz.load_from(oz, keys=("cv", "bv"))
+    oz.call("orc_apply_boundary_conditions")
+    gz.ctx.boundary_conditions()
+    for k in ("bv", "cv"):
+        assert rel_err(gz.get(k), oz[k][: gz.t[k].shape[0]], momentum=()) <= 1e-14, k
+
+
+@pytest.mark.parametrize("shape", [(9, 7, 5), (5, 9, 6), (33, 5, 5)])
+def test_properties_shell_covers_what_the_update_leaves(shape):
+    """After a step every property of the padded block is that of its final
+    state: the update's nodes and the shell's together are all of them."""
+    n, ny, nz = shape
+    mech = mechanism.load("li2004")
+    case = cases.perturbed(cases.mix_wave(mech, n, ny=ny, nz=nz, scheme=52, dt=1e-9), seed=2,
+                           amp=1e-3)
+    gz = GpuZone(case)
+    gz.initialize()
+    gz.ctx.rk3_step()
+    keys = ("mul", "gamma", "acoustic_speed", "thermal_conductivity", "rho_D")
+    out = {k: gz.get(k).copy() for k in keys}
+    gz.ctx.properties()
+    for k in keys:
+        assert np.allclose(out[k], gz.get(k), rtol=1e-14, atol=0), k
