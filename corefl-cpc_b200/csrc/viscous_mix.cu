@@ -5,7 +5,11 @@
 // conductivity, mixture-averaged species diffusion rho D_k (grad Y_k -
 // Y_k grad W / W) with the correction velocity, and the enthalpy flux
 // sum h_k J_k at the face temperature), and compute_dFv_dx / dGv_dy / dHv_dz
-// (:75-127).  Same face tiling as viscous_air.cu; the face fluxes of all
+// (:75-127).  Bound by the latency of its loads (L1 and L2 hits): the species
+// are taken in two loops that hold nothing a species, 128 registers and two
+// CTAs an SM; with every species in registers it took 178, one CTA (8 warps) an
+// SM, and 725 us instead of 389 on a 128 x 65 x 63 block.  Three CTAs at 80
+// registers spill and take 433.  Same face tiling as viscous_air.cu; the face fluxes of all
 // 4 + NS viscous components stay in shared memory.  With gradp set the
 // diffusion driving force also carries the pressure-gradient term
 // (W/W_k - 1) Y_k grad(xi).grad(p) / p of gradPInDiffusionFlux (reference
@@ -32,7 +36,7 @@ struct VisMixTile {
 }  // namespace
 
 template <int DIR, int NS>
-__global__ void __launch_bounds__(256) viscous_mix_flux_diff(Zone z, const __grid_constant__ Thermo thermo,
+__global__ void __launch_bounds__(256, 2) viscous_mix_flux_diff(Zone z, const __grid_constant__ Thermo thermo,
                                                              int gradp) {
   using T = VisMixTile<DIR, NS>;
   constexpr int TN = T::TN, C = T::C, NF = T::NF;
@@ -107,60 +111,58 @@ __global__ void __launch_bounds__(256) viscous_mix_flux_diff(Zone z, const __gri
     const double um = 0.5 * (pv[id + sz] + pv[idn + sz]);
     const double vm = 0.5 * (pv[id + 2 * sz] + pv[idn + 2 * sz]);
     const double wm = 0.5 * (pv[id + 3 * sz] + pv[idn + 3 * sz]);
-    const double t_x = dd[3][0] * gm[0] + dd[3][1] * gm[3] + dd[3][2] * gm[6];
-    const double t_y = dd[3][0] * gm[1] + dd[3][1] * gm[4] + dd[3][2] * gm[7];
-    const double t_z = dd[3][0] * gm[2] + dd[3][1] * gm[5] + dd[3][2] * gm[8];
-    const double conductivity = 0.5 * (z.thermal_conductivity[id] + z.thermal_conductivity[idn]);
-    double f3 = um * f0 + vm * f1 + wm * f2 + conductivity * (gk0 * t_x + gk1 * t_y + gk2 * t_z);
-
-    // species diffusion with the correction velocity (mixture-averaged)
-    const double *y = z.sv;
-    double yk[NS], diffusivity[NS], ddf[NS];
-    double sum_grad_over_w = 0, sum_rhoDkYk = 0, correction = 0, mw_tot = 0;
+    // grad(xi_normal) J . grad of a scalar from its three differences
+    double M[3];
 #pragma unroll
+    for (int a = 0; a < 3; ++a) M[a] = fma(gk0, gm[3 * a], fma(gk1, gm[3 * a + 1], gk2 * gm[3 * a + 2]));
+    const double conductivity = 0.5 * (z.thermal_conductivity[id] + z.thermal_conductivity[idn]);
+    double f3 = um * f0 + vm * f1 + wm * f2 +
+                conductivity * fma(M[0], dd[3][0], fma(M[1], dd[3][1], M[2] * dd[3][2]));
+    auto normal_grad = [&](const double *f) {
+      const double dn = f[idn] - f[id];
+      const double da = 0.25 * ((f[id + sa] - f[id - sa]) + (f[idn + sa] - f[idn - sa]));
+      const double db = 0.25 * ((f[id + sb] - f[id - sb]) + (f[idn + sb] - f[idn - sb]));
+      return fma(M[DIR], dn, fma(M[DA], da, M[DB] * db));
+    };
+
+    // species diffusion with the correction velocity (mixture-averaged): the
+    // sums over the species first, each species' gradient waiting in its slot
+    // of the flux buffer, then the fluxes; the mass fraction and diffusivity
+    // of a species are read again (from L1) rather than held
+    const double *y = z.sv;
+    double sum_grad_over_w = 0, sum_rhoDkYk = 0, correction = 0, imw_tot = 0, sum_over_w = 0;
+#pragma unroll 3
     for (int l = 0; l < NS; ++l) {
-      const double *yl = y + l * sz;
-      yk[l] = 0.5 * (yl[id] + yl[idn]);
-      diffusivity[l] = 0.5 * (z.rho_D[id + l * sz] + z.rho_D[idn + l * sz]);
-      double d3[3];
-      d3[DIR] = yl[idn] - yl[id];
-      d3[DA] = 0.25 * (yl[id + sa] - yl[id - sa] + yl[idn + sa] - yl[idn - sa]);
-      d3[DB] = 0.25 * (yl[id + sb] - yl[id - sb] + yl[idn + sb] - yl[idn - sb]);
-      const double y_x = d3[0] * gm[0] + d3[1] * gm[3] + d3[2] * gm[6];
-      const double y_y = d3[0] * gm[1] + d3[1] * gm[4] + d3[2] * gm[7];
-      const double y_z = d3[0] * gm[2] + d3[1] * gm[5] + d3[2] * gm[8];
-      const double gy = gk0 * y_x + gk1 * y_y + gk2 * y_z;
-      ddf[l] = gy;
-      correction += diffusivity[l] * gy;
-      sum_grad_over_w += gy * th->imw[l];
-      mw_tot += yk[l] * th->imw[l];
-      sum_rhoDkYk += diffusivity[l] * yk[l];
+      const double *yl = y + l * sz, *dl = z.rho_D + l * sz;
+      const double yk = 0.5 * (yl[id] + yl[idn]), dk = 0.5 * (dl[id] + dl[idn]);
+      const double gy = normal_grad(yl), w = th->imw[l], dy = dk * yk;
+      sflx[T::sfl(4 + l, c, t)] = gy;
+      correction = fma(dk, gy, correction);
+      sum_grad_over_w = fma(gy, w, sum_grad_over_w);
+      imw_tot = fma(yk, w, imw_tot);
+      sum_rhoDkYk += dy;
+      sum_over_w = fma(dy, w, sum_over_w);
     }
-    mw_tot = 1.0 / mw_tot;
-    correction -= mw_tot * sum_rhoDkYk * sum_grad_over_w;
+    const double mw_tot = 1.0 / imw_tot, mg = mw_tot * sum_grad_over_w;
+    correction -= sum_rhoDkYk * mg;
+    double gp = 0;
     if (gradp) {
       const double *pp = pv + 4 * sz;
-      double d3[3];
-      d3[DIR] = pp[idn] - pp[id];
-      d3[DA] = 0.25 * (pp[id + sa] - pp[id - sa] + pp[idn + sa] - pp[idn - sa]);
-      d3[DB] = 0.25 * (pp[id + sb] - pp[id - sb] + pp[idn + sb] - pp[idn - sb]);
-      const double p_x = d3[0] * gm[0] + d3[1] * gm[3] + d3[2] * gm[6];
-      const double p_y = d3[0] * gm[1] + d3[1] * gm[4] + d3[2] * gm[7];
-      const double p_z = d3[0] * gm[2] + d3[1] * gm[5] + d3[2] * gm[8];
-      const double gp = (gk0 * p_x + gk1 * p_y + gk2 * p_z) / (0.5 * (pp[idn] + pp[id]));
-#pragma unroll
-      for (int l = 0; l < NS; ++l) {
-        ddf[l] += (mw_tot * th->imw[l] - 1) * yk[l] * gp;
-        correction += (mw_tot * th->imw[l] - 1) * yk[l] * gp * diffusivity[l];
-      }
+      gp = normal_grad(pp) / (0.5 * (pp[idn] + pp[id]));
+      correction = fma(gp, fma(mw_tot, sum_over_w, -sum_rhoDkYk), correction);
     }
-    double h[NS], cp_unused[NS];
-    enthalpy_cp_ns<NS>(th, 0.5 * (pv[id + 5 * sz] + pv[idn + 5 * sz]), h, cp_unused);
-#pragma unroll
+    const double tf = 0.5 * (pv[id + 5 * sz] + pv[idn + 5 * sz]);
+#pragma unroll 3
     for (int l = 0; l < NS; ++l) {
-      const double flux = diffusivity[l] * (ddf[l] - mw_tot * yk[l] * sum_grad_over_w) - yk[l] * correction;
+      const double *yl = y + l * sz, *dl = z.rho_D + l * sz;
+      const double yk = 0.5 * (yl[id] + yl[idn]), dk = 0.5 * (dl[id] + dl[idn]);
+      // gy - Y mg, with the pressure term Y (mw/W - 1) gp
+      const double drive = sflx[T::sfl(4 + l, c, t)] - yk * (mg - (mw_tot * th->imw[l] - 1) * gp);
+      const double flux = dk * drive - yk * correction;
+      double h, cp;
+      enthalpy_cp_one(th, l, tf, h, cp);
       sflx[T::sfl(4 + l, c, t)] = flux;
-      f3 += h[l] * flux;
+      f3 = fma(h, flux, f3);
     }
     sflx[T::sfl(0, c, t)] = f0;
     sflx[T::sfl(1, c, t)] = f1;
@@ -175,7 +177,8 @@ __global__ void __launch_bounds__(256) viscous_mix_flux_diff(Zone z, const __gri
     if (cbase + c >= ncol_max || a > m - 1) continue;
     const int64_t iq = node_idx(0, c, a);
 #pragma unroll
-    for (int v = 0; v < T::NVF; ++v) z.dq[iq + (v + 1) * szq] += sflx[T::sfl(v, c, t + 1)] - sflx[T::sfl(v, c, t)];
+    for (int v = 0; v < T::NVF; ++v)
+      red_add(z.dq + iq + (v + 1) * szq, sflx[T::sfl(v, c, t + 1)] - sflx[T::sfl(v, c, t)]);
   }
 }
 
