@@ -17,31 +17,26 @@
 
 namespace cfk {
 
+// minmod with gxl::sgn, which returns +1 for zero: 0.5 (sgn a + sgn b)
+// min(|a|, |b|) written without its integer-to-double conversion.
 __device__ __forceinline__ double minmod_ref(double a, double b) {
-  // gxl::sgn returns +1 for zero
-  const int sa = a < 0 ? -1 : 1, sb = b < 0 ? -1 : 1;
-  return 0.5 * (sa + sb) * fmin(fabs(a), fabs(b));
+  const bool na = a < 0, nb = b < 0;
+  const double m = fmin(fabs(a), fabs(b));
+  return na != nb ? 0.0 : na ? -m : m;
 }
 
-// v0..v3: one primitive variable at nodes i-1, i, i+1, i+2 -> states at i+1/2
+// v0..v3: one primitive variable at nodes i-1, i, i+1, i+2 -> states at i+1/2.
+// minmod is symmetric, so MUSCL's two limited differences of a side are one
+// value and its (1 - kappa) and (1 + kappa) shares add up to NND2's half.
 template <int RECON>
 __device__ __forceinline__ void reconstruct_var(double v0, double v1, double v2, double v3, double &l, double &r) {
-  if (RECON == 2) {
-    constexpr double kappa = 1.0 / 3.0;
-    const double delta_i = v1 - v0, delta_i1 = v2 - v1, delta_i2 = v3 - v2;
-    const double delta_neg_l = minmod_ref(delta_i, delta_i1);
-    const double delta_pos_l = minmod_ref(delta_i1, delta_i);
-    const double delta_neg_r = minmod_ref(delta_i1, delta_i2);
-    const double delta_pos_r = minmod_ref(delta_i2, delta_i1);
-    l = v1 + 0.25 * ((1 - kappa) * delta_neg_l + (1 + kappa) * delta_pos_l);
-    r = v2 - 0.25 * ((1 - kappa) * delta_pos_r + (1 + kappa) * delta_neg_r);
-  } else if (RECON == 3) {
-    const double delta_i = v1 - v0, delta_i1 = v2 - v1, delta_i2 = v3 - v2;
-    l = v1 + 0.5 * minmod_ref(delta_i, delta_i1);
-    r = v2 - 0.5 * minmod_ref(delta_i1, delta_i2);
-  } else {
+  if (RECON == 1) {
     l = v1;
     r = v2;
+  } else {
+    const double delta_i = v1 - v0, delta_i1 = v2 - v1, delta_i2 = v3 - v2;
+    l = fma(0.5, minmod_ref(delta_i, delta_i1), v1);
+    r = fma(-0.5, minmod_ref(delta_i1, delta_i2), v2);
   }
 }
 
@@ -55,17 +50,18 @@ __device__ __forceinline__ void ausm_plus_air(const double *pl, const double *pr
   const double k1 = 0.5 * (jac[0] * m[0][0] + jac[1] * m[1][0]);
   const double k2 = 0.5 * (jac[0] * m[0][1] + jac[1] * m[1][1]);
   const double k3 = 0.5 * (jac[0] * m[0][2] + jac[1] * m[1][2]);
-  const double grad_k_div_jac = sqrt(k1 * k1 + k2 * k2 + k3 * k3);
-  const double ul = (k1 * pl[1] + k2 * pl[2] + k3 * pl[3]) / grad_k_div_jac;
-  const double ur = (k1 * pr[1] + k2 * pr[2] + k3 * pr[3]) / grad_k_div_jac;
+  const double kk = k1 * k1 + k2 * k2 + k3 * k3, ik = rsqrt(kk), grad_k_div_jac = kk * ik;
+  const double irho_l = rcp_nr(pl[0]), irho_r = rcp_nr(pr[0]);
+  const double ul = (k1 * pl[1] + k2 * pl[2] + k3 * pl[3]) * ik;
+  const double ur = (k1 * pr[1] + k2 * pr[2] + k3 * pr[3]) * ik;
   const double p_l = pl[4], p_r = pr[4], rho_l = pl[0], rho_r = pr[0];
-  const double c = 0.5 * (sqrt(kGammaAir * p_l / rho_l) + sqrt(kGammaAir * p_r / rho_r));
-  const double mach_l = ul / c, mach_r = ur / c;
+  const double c = 0.5 * (sqrt(kGammaAir * p_l * irho_l) + sqrt(kGammaAir * p_r * irho_r));
+  const double ic = rcp_nr(c), mach_l = ul * ic, mach_r = ur * ic;
   double mlp, mrn, plp, prn;
   constexpr double alpha = 3 / 16.0;
   if (fabs(mach_l) > 1) {
     mlp = 0.5 * (mach_l + fabs(mach_l));
-    plp = mlp / mach_l;
+    plp = mach_l > 0 ? 1.0 : 0.0;  // mlp / mach_l
   } else {
     const double a = (mach_l + 1) * (mach_l + 1) * 0.25;
     const double b = (mach_l * mach_l - 1) * (mach_l * mach_l - 1);
@@ -74,7 +70,7 @@ __device__ __forceinline__ void ausm_plus_air(const double *pl, const double *pr
   }
   if (fabs(mach_r) > 1) {
     mrn = 0.5 * (mach_r - fabs(mach_r));
-    prn = mrn / mach_r;
+    prn = mach_r < 0 ? 1.0 : 0.0;  // mrn / mach_r
   } else {
     const double a = (mach_r - 1) * (mach_r - 1) * 0.25;
     const double b = (mach_r * mach_r - 1) * (mach_r * mach_r - 1);
@@ -92,31 +88,34 @@ __device__ __forceinline__ void ausm_plus_air(const double *pl, const double *pr
   fc[1] = coeff * pv[1] + p_coeff * k1;
   fc[2] = coeff * pv[2] + p_coeff * k2;
   fc[3] = coeff * pv[3] + p_coeff * k3;
-  fc[4] = coeff * (pv[5] + pv[4]) / pv[0];
+  fc[4] = coeff * (pv[5] + pv[4]) * (mass_flux_half >= 0 ? irho_l : irho_r);
 }
 
 __device__ __forceinline__ void hllc_air(const double *pl, const double *pr, const double m[2][3], const double jac[2],
                                          double *fc) {
-  const double rl_c = sqrt(pl[0]) / (sqrt(pl[0]) + sqrt(pr[0]));
-  const double rr_c = sqrt(pr[0]) / (sqrt(pl[0]) + sqrt(pr[0]));
+  const double sql = sqrt(pl[0]), sqr = sqrt(pr[0]), isum = rcp_nr(sql + sqr);
+  const double rl_c = sql * isum;
+  const double rr_c = sqr * isum;
+  const double irho_l = rcp_nr(pl[0]), irho_r = rcp_nr(pr[0]);
   const double u_tilde = pl[1] * rl_c + pr[1] * rr_c;
   const double v_tilde = pl[2] * rl_c + pr[2] * rr_c;
   const double w_tilde = pl[3] * rl_c + pr[3] * rr_c;
   constexpr double gamma = kGammaAir;
-  const double hl = (pl[5] + pl[4]) / pl[0];
-  const double hr = (pr[5] + pr[4]) / pr[0];
+  const double hl = (pl[5] + pl[4]) * irho_l;
+  const double hr = (pr[5] + pr[4]) * irho_r;
   const double h_tilde = hl * rl_c + hr * rr_c;
   const double ek_tilde = 0.5 * (u_tilde * u_tilde + v_tilde * v_tilde + w_tilde * w_tilde);
   const double c_tilde = sqrt((gamma - 1) * (h_tilde - ek_tilde));
   const double kx = 0.5 * (m[0][0] + m[1][0]);
   const double ky = 0.5 * (m[0][1] + m[1][1]);
   const double kz = 0.5 * (m[0][2] + m[1][2]);
-  const double gradK = sqrt(kx * kx + ky * ky + kz * kz);
-  const double U_tilde_bar = (kx * u_tilde + ky * v_tilde + kz * w_tilde) / gradK;
+  const double k2 = kx * kx + ky * ky + kz * kz, igradK = rsqrt(k2), gradK = k2 * igradK;
+  const double U_tilde_bar = (kx * u_tilde + ky * v_tilde + kz * w_tilde) * igradK;
   const double jac_ave = 0.5 * (jac[0] + jac[1]);
   const double Ul = kx * pl[1] + ky * pl[2] + kz * pl[3];
-  const double cl = sqrt(kGammaAir * pl[4] / pl[0]);
-  const double sl = fmin(Ul / gradK - cl, U_tilde_bar - c_tilde);
+  const double cl = sqrt(kGammaAir * pl[4] * irho_l);
+  const double ul = Ul * igradK;
+  const double sl = fmin(ul - cl, U_tilde_bar - c_tilde);
   if (sl >= 0) {
     const double rhoUk = pl[0] * Ul;
     fc[0] = jac_ave * rhoUk;
@@ -127,8 +126,9 @@ __device__ __forceinline__ void hllc_air(const double *pl, const double *pr, con
     return;
   }
   const double Ur = kx * pr[1] + ky * pr[2] + kz * pr[3];
-  const double cr = sqrt(kGammaAir * pr[4] / pr[0]);
-  const double sr = fmax(Ur / gradK + cr, U_tilde_bar + c_tilde);
+  const double cr = sqrt(kGammaAir * pr[4] * irho_r);
+  const double ur = Ur * igradK;
+  const double sr = fmax(ur + cr, U_tilde_bar + c_tilde);
   if (sr < 0) {
     const double rhoUk = pr[0] * Ur;
     fc[0] = jac_ave * rhoUk;
@@ -138,20 +138,20 @@ __device__ __forceinline__ void hllc_air(const double *pl, const double *pr, con
     fc[4] = jac_ave * ((pr[5] + pr[4]) * Ur);
     return;
   }
-  const double sm = ((pr[0] * Ur * (sr - Ur / gradK) - pl[0] * Ul * (sl - Ul / gradK)) / gradK + pl[4] - pr[4]) /
-                    (pr[0] * (sr - Ur / gradK) - pl[0] * (sl - Ul / gradK));
-  const double pm = pl[0] * (sl - Ul / gradK) * (sm - Ul / gradK) + pl[4];
+  const double sm = ((pr[0] * Ur * (sr - ur) - pl[0] * Ul * (sl - ul)) * igradK + pl[4] - pr[4]) *
+                    rcp_nr(pr[0] * (sr - ur) - pl[0] * (sl - ul));
+  const double pm = pl[0] * (sl - ul) * (sm - ul) + pl[4];
   const bool left = sm >= 0;
   const double *ps = left ? pl : pr;
-  const double ss = left ? sl : sr, Us = left ? Ul : Ur;
-  const double pCoeff = 1.0 / (ss - sm);
+  const double ss = left ? sl : sr, Us = left ? Ul : Ur, irho = left ? irho_l : irho_r;
+  const double pCoeff = rcp_nr(ss - sm);
   const double QCoeff = jac_ave * pCoeff * sm * (ss * gradK - Us) * ps[0];
   fc[0] = QCoeff;
   const double dP = (ss * pm - sm * ps[4]) * pCoeff * jac_ave;
   fc[1] = QCoeff * ps[1] + dP * kx;
   fc[2] = QCoeff * ps[2] + dP * ky;
   fc[3] = QCoeff * ps[3] + dP * kz;
-  fc[4] = QCoeff * ps[5] / ps[0] + pCoeff * jac_ave * (ss * pm * sm * gradK - sm * ps[4] * Us);
+  fc[4] = QCoeff * ps[5] * irho + pCoeff * jac_ave * (ss * pm * sm * gradK - sm * ps[4] * Us);
 }
 
 __device__ __forceinline__ void lax_friedrichs_air(const double *pl, const double *pr, const double m[2][3],
@@ -162,8 +162,8 @@ __device__ __forceinline__ void lax_friedrichs_air(const double *pl, const doubl
   const double gradK = sqrt(kx * kx + ky * ky + kz * kz);
   const double Ukl = pl[1] * kx + pl[2] * ky + pl[3] * kz;
   const double Ukr = pr[1] * kx + pr[2] * ky + pr[3] * kz;
-  const double cl = sqrt(kGammaAir * pl[4] / pl[0]);
-  const double cr = sqrt(kGammaAir * pr[4] / pr[0]);
+  const double cl = sqrt(kGammaAir * pl[4] * rcp_nr(pl[0]));
+  const double cr = sqrt(kGammaAir * pr[4] * rcp_nr(pr[0]));
   const double spectral_radius = fmax(fabs(Ukl) + cl * gradK, fabs(Ukr) + cr * gradK);
   const double half_jac_ave = 0.5 * 0.5 * (jac[0] + jac[1]);
   const double rhoUl = pl[0] * Ukl;
@@ -187,9 +187,9 @@ __device__ __forceinline__ double entropy_fix_delta_air(double rho, double u, do
   const double kx = sqrt(mt[0] * mt[0] + mt[1] * mt[1] + mt[2] * mt[2]);
   const double ky = sqrt(mt[3] * mt[3] + mt[4] * mt[4] + mt[5] * mt[5]);
   const double kz = sqrt(mt[6] * mt[6] + mt[7] * mt[7] + mt[8] * mt[8]);
-  const double acoustic_speed = sqrt(kGammaAir * p / rho);
+  const double acoustic_speed = sqrt(kGammaAir * p * rcp_nr(rho));
   if (dim == 2) return factor * (U + V + acoustic_speed * 0.5 * (kx + ky));
-  return factor * (U + V + W + acoustic_speed * (kx + ky + kz) / 3.0);
+  return factor * (U + V + W + acoustic_speed * (kx + ky + kz) * (1.0 / 3.0));
 }
 
 __device__ __forceinline__ void roe_air(const double *pl, const double *pr, const double m[2][3], const double jac[2],
@@ -214,34 +214,34 @@ __device__ __forceinline__ void roe_air(const double *pl, const double *pr, cons
   fc[4] += 0.5 * Uk * (pr[4] + pr[5]);
 
   const double dl = sqrt(pl[0]), dr = sqrt(pr[0]);
-  const double inv_denominator = 1.0 / (dl + dr);
+  const double inv_denominator = rcp_nr(dl + dr);
   const double u = (dl * pl[1] + dr * pr[1]) * inv_denominator;
   const double v = (dl * pl[2] + dr * pr[2]) * inv_denominator;
   const double w = (dl * pl[3] + dr * pr[3]) * inv_denominator;
   const double ek = 0.5 * (u * u + v * v + w * w);
-  const double hl = (pl[5] + pl[4]) / pl[0];
-  const double hr = (pr[5] + pr[4]) / pr[0];
+  const double hl = (pl[5] + pl[4]) * rcp_nr(pl[0]);
+  const double hr = (pr[5] + pr[4]) * rcp_nr(pr[0]);
   const double h = (dl * hl + dr * hr) * inv_denominator;
   constexpr double gamma = kGammaAir;
-  const double c = sqrt((gamma - 1) * (h - ek));
+  const double c2_ = (gamma - 1) * (h - ek), ic = rsqrt(c2_), c = c2_ * ic;
 
   double kx = 0.5 * (m[0][0] + m[1][0]);
   double ky = 0.5 * (m[0][1] + m[1][1]);
   double kz = 0.5 * (m[0][2] + m[1][2]);
-  const double gradK = sqrt(kx * kx + ky * ky + kz * kz);
+  const double k2 = kx * kx + ky * ky + kz * kz, igradK = rsqrt(k2), gradK = k2 * igradK;
   double Ukk = kx * u + ky * v + kz * w;
   double ch[3] = {Ukk - gradK * c, Ukk, Ukk + gradK * c};
   const double entropy_fix_delta_ave = 0.5 * (delta[0] + delta[1]);
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     double cc = fabs(ch[q]);
-    if (cc < entropy_fix_delta_ave) cc = 0.5 * (cc * cc / entropy_fix_delta_ave + entropy_fix_delta_ave);
+    if (cc < entropy_fix_delta_ave) cc = 0.5 * (cc * cc * rcp_nr(entropy_fix_delta_ave) + entropy_fix_delta_ave);
     ch[q] = cc;
   }
-  kx /= gradK;
-  ky /= gradK;
-  kz /= gradK;
-  Ukk /= gradK;
+  kx *= igradK;
+  ky *= igradK;
+  kz *= igradK;
+  Ukk *= igradK;
 
   const double jac_ave = 0.5 * (jac[0] + jac[1]);
   double dq[5];
@@ -250,14 +250,14 @@ __device__ __forceinline__ void roe_air(const double *pl, const double *pr, cons
   for (int l = 1; l < 4; ++l) dq[l] = jac_ave * (pr[0] * pr[l] - pl[0] * pl[l]);
   dq[4] = jac_ave * (pr[5] - pl[5]);
 
-  double c1 = (gamma - 1) * (ek * dq[0] - u * dq[1] - v * dq[2] - w * dq[3] + dq[4]) / (c * c);
-  double c2 = (kx * dq[1] + ky * dq[2] + kz * dq[3] - Ukk * dq[0]) / c;
+  double c1 = (gamma - 1) * (ek * dq[0] - u * dq[1] - v * dq[2] - w * dq[3] + dq[4]) * (ic * ic);
+  double c2 = (kx * dq[1] + ky * dq[2] + kz * dq[3] - Ukk * dq[0]) * ic;
   double c3 = dq[0] - c1;
   double LDq[5];
   LDq[0] = 0.5 * (c1 - c2);
-  LDq[1] = kx * c3 - ((kz * v - ky * w) * dq[0] - kz * dq[2] + ky * dq[3]) / c;
-  LDq[2] = ky * c3 - ((kx * w - kz * u) * dq[0] - kx * dq[3] + kz * dq[1]) / c;
-  LDq[3] = kz * c3 - ((ky * u - kx * v) * dq[0] - ky * dq[1] + kx * dq[2]) / c;
+  LDq[1] = kx * c3 - ((kz * v - ky * w) * dq[0] - kz * dq[2] + ky * dq[3]) * ic;
+  LDq[2] = ky * c3 - ((kx * w - kz * u) * dq[0] - kx * dq[3] + kz * dq[1]) * ic;
+  LDq[3] = kz * c3 - ((ky * u - kx * v) * dq[0] - ky * dq[1] + kx * dq[2]) * ic;
   LDq[4] = 0.5 * (c1 + c2);
 
   double b[5];
@@ -275,7 +275,7 @@ __device__ __forceinline__ void roe_air(const double *pl, const double *pr, cons
   fc[1] += 0.5 * (u * c1 + kx * c2 - c * (kz * b[2] - ky * b[3]));
   fc[2] += 0.5 * (v * c1 + ky * c2 - c * (kx * b[3] - kz * b[1]));
   fc[3] += 0.5 * (w * c1 + kz * c2 - c * (ky * b[1] - kx * b[2]));
-  fc[4] += 0.5 * (h * c1 + Ukk * c2 - c * c * c0 / (gamma - 1) +
+  fc[4] += 0.5 * (h * c1 + Ukk * c2 - c * c * c0 * (1 / (gamma - 1)) +
                   c * ((kz * v - ky * w) * b[1] + (kx * w - kz * u) * b[2] + (ky * u - kx * v) * b[3]) + c3);
 }
 

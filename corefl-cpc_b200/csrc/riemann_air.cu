@@ -14,8 +14,13 @@
 //           points, reads the two nodes' metric row and Jacobian (coalesced
 //           along i) and evaluates the Riemann flux into shared memory;
 //   diff  — dq(n) -= F(n+1/2) - F(n-1/2).
-// Memory-bound: per node and direction it reads bv[5], metric[3], jac (Roe:
-// metric[9]) and read-modify-writes dq[5].
+// Per node and direction it reads bv[5], metric[3], jac (Roe: metric[9]) and
+// adds to dq[5].  Bound by FP64 issue and latency, not by memory: small tiles,
+// one or two faces a thread of a 128-thread CTA, six CTAs an SM, overlap their
+// phases.  Roe + MUSCL on a 193 x 101 x 89 block, three sweeps: 727 us with
+// 256-thread CTAs of 124 x 2 and 28 x 32 nodes, integer-to-double conversions
+// in minmod and some fifteen divisions a face; 305 now (at five CTAs 311; 31
+// x 4 and 7 x 32: 333; 63 x 2 and 15 x 32: 373; 124 x 1 and 31 x 32: 445).
 #include "cfk_common.cuh"
 #include "riemann.cuh"
 
@@ -25,12 +30,12 @@ namespace {
 
 template <int DIR, int SCH>
 struct PvTile {
-  static constexpr int TN = DIR == 0 ? 124 : 28;  // nodes per column
-  static constexpr int C = DIR == 0 ? 2 : 32;     // columns per CTA
+  static constexpr int TN = DIR == 0 ? 63 : 15;  // nodes per column
+  static constexpr int C = DIR == 0 ? 2 : 16;    // columns per CTA
   static constexpr int NF = TN + 1;               // faces per column
   static constexpr int NPT = TN + 4;              // staged points per column (i-2 .. i+TN+1)
   static constexpr int NQ = SCH == 2 ? 6 : 5;     // rho, u, v, w, p (+ entropy-fix width)
-  static constexpr int NT = 256;
+  static constexpr int NT = 128;
   __device__ static int spt(int q, int c, int t) {
     return DIR == 0 ? (q * C + c) * NPT + t : (q * NPT + t) * C + c;
   }
@@ -43,7 +48,7 @@ struct PvTile {
 }  // namespace
 
 template <int DIR, int SCH, int RECON>
-__global__ void __launch_bounds__(256) pv_air_flux_diff(Zone z, int dim, double entropy_fix_factor) {
+__global__ void __launch_bounds__(128, 6) pv_air_flux_diff(Zone z, int dim, double entropy_fix_factor) {
   using T = PvTile<DIR, SCH>;
   constexpr int TN = T::TN, C = T::C, NF = T::NF, NPT = T::NPT;
   extern __shared__ double sm[];
@@ -141,7 +146,7 @@ __global__ void __launch_bounds__(256) pv_air_flux_diff(Zone z, int dim, double 
     if (cbase + c >= ncol_max || a >= m) continue;
     const int64_t iq = node_idx(0, c, a);
 #pragma unroll
-    for (int l = 0; l < 5; ++l) z.dq[iq + l * szq] -= sflx[T::sfl(l, c, t + 1)] - sflx[T::sfl(l, c, t)];
+    for (int l = 0; l < 5; ++l) red_add(z.dq + iq + l * szq, sflx[T::sfl(l, c, t)] - sflx[T::sfl(l, c, t + 1)]);
   }
 }
 

@@ -41,3 +41,18 @@ def test_pv_inviscid_flux_perturbed_single_call(scheme):
     gz.ctx.inviscid()
     oz.call("orc_compute_inviscid_flux")
     assert rel_err(gz.get("dq"), oz["dq"]) <= 1e-11
+
+
+@pytest.mark.parametrize("scheme", [2, 4])
+@pytest.mark.parametrize("n, ny, nz", [(63, 15, 16), (64, 16, 15), (65, 31, 9)])
+def test_pv_inviscid_flux_tile_edges(scheme, n, ny, nz):
+    """Extents at the tiles' edges (63 nodes along i, 15 along j and k, 16
+    columns); the bar of the single call above."""
+    case = cases.perturbed(cases.sine_wave(n=n, ny=ny, nz=nz, scheme=scheme, viscous=False, amp=0.1), seed=4, amp=0.2)
+    oz = pyoracle.OracleZone(case)
+    oz.initialize()
+    gz = GpuZone(case)
+    gz.initialize()
+    gz.ctx.inviscid()
+    oz.call("orc_compute_inviscid_flux")
+    assert rel_err(gz.get("dq"), oz["dq"]) <= 1e-11
