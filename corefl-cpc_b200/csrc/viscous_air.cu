@@ -10,17 +10,18 @@
 
 namespace cfk {
 
-// All three directions in one kernel: a CTA owns a 32 x 8 tile of (i, j)
+// All three directions in one kernel: a CTA owns a 32 x 4 tile of (i, j)
 // columns and marches along k through a chunk of planes, keeping two planes
 // of per-node values (u, v, w, T, mu, J, metric) with a one-node halo in
 // shared memory plus the k-differences f(k+1) - f(k-1) of the current plane.
 // Per plane it computes the x and y faces of the plane and the z face above
 // each node; the z face below comes from the previous plane.  dq gets the x,
 // y and z differences added in that order, the order of the reference's
-// per-direction derivative kernels.  Every node's inputs are read from HBM
+// per-direction derivative kernels (the ring variant adds their sum).  Every node's inputs are read from HBM
 // once per stage and dq once instead of three times.
 namespace {
-constexpr int kFX = 32, kFY = 8, kFZ = 32;     // tile and planes per chunk
+constexpr int kFX = 32, kFY = 4;               // tile; the planes of a chunk: viscous_chunk
+constexpr int kCtas = 3;                       // CTAs an SM of the ring form
 constexpr int kPX = kFX + 2, kPY = kFY + 2;    // staged points per plane
 constexpr int kNV = 15;                        // u v w T mu J metric[9]
 constexpr int kFT = kFX * kFY;                 // threads
@@ -99,17 +100,17 @@ __device__ __forceinline__ void staged_face(const FusedSmem &S, int sa, int pa, 
 }
 }  // namespace
 
-__global__ void __launch_bounds__(kFT, 2) viscous_air_fused(Zone z, double Pr) {
+__global__ void __launch_bounds__(kFT, 2) viscous_air_fused(Zone z, double Pr, int planes) {
   extern __shared__ __align__(16) double fsm[];
   const double cp_pr = kCpAir / Pr;
   FusedSmem &S = *reinterpret_cast<FusedSmem *>(fsm);
   const Dims d = z.d;
   const int g = d.ngg;
   const int64_t sz = d.plane(g), szq = d.plane(0);
-  const int i0 = blockIdx.x * kFX, j0 = blockIdx.y * kFY, k0 = blockIdx.z * kFZ;
+  const int i0 = blockIdx.x * kFX, j0 = blockIdx.y * kFY, k0 = blockIdx.z * planes;
   const int tx = threadIdx.x % kFX, ty = threadIdx.x / kFX;
   const bool three_d = d.mz > 1;
-  const int k_end = min(k0 + kFZ, d.mz);
+  const int k_end = min(k0 + planes, d.mz);
 
   // per-thread share of a plane's staged points: p = threadIdx.x, + kFT
   auto point_ok = [&](int p, int &px, int &py) {
@@ -229,14 +230,14 @@ __global__ void __launch_bounds__(kFT, 2) viscous_air_fused(Zone z, double Pr) {
   }
 }
 
-// Ring variant: the same tile, march and arithmetic, with only the dynamic
+// Ring variant: the same tile and march, with only the dynamic
 // values (u, v, w, T, mu) staged in shared memory, in a ring of three plane
 // slots filled by cp.async: plane k+2 is requested before the faces of plane
 // k are computed and lands while they run, so the loads never stall a warp.
-// The metric and J (read-only) come through L1 from global memory.  70 KB of
-// shared memory per CTA, two CTAs per SM, two barriers per plane.  The face
-// flux is term for term that of staged_face (the compiler may contract its
-// products into FMAs differently, so the two agree to the last bits).
+// The metric and J (read-only) come from global memory into registers.  41 KB
+// of shared memory per CTA, two barriers per plane.  The face flux is term for
+// term that of staged_face, and the three differences are summed before they
+// are added to dq, so the two agree to the last bits.
 namespace {
 constexpr int kRV = 5;  // u v w T mu
 
@@ -257,12 +258,10 @@ __device__ __forceinline__ void prefetch_l2(const double *p) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// staged_face with the metric and J of the two nodes (global indices ida, idb) read from global memory.
+// staged_face with the metric [0..8] and J [9] of the two nodes in registers.
 template <int DIR>
-__device__ __forceinline__ void ring_face(const RingSmem &S, const double *__restrict__ met,
-                                          const double *__restrict__ jac, int64_t sz, int sa, int pa, int qa,
-                                          int64_t ida, int sb, int pb, int qb, int64_t idb, double cp_pr,
-                                          double F[4]) {
+__device__ __forceinline__ void ring_face(const RingSmem &S, int sa, int pa, int qa, const double (&ma)[10], int sb,
+                                          int pb, int qb, const double (&mb)[10], double cp_pr, double (&F)[4]) {
   const auto &A = S.dyn[sa];
   const auto &B = S.dyn[sb];
   auto tdiff = [&](const double (&p)[kRV][kPY][kPX], int D, int q, int px, int py) -> double {
@@ -273,7 +272,7 @@ __device__ __forceinline__ void ring_face(const RingSmem &S, const double *__res
   constexpr int TLO = DIR == 0 ? 1 : 0, THI = DIR == 2 ? 1 : 2;
   double gm[9];
 #pragma unroll
-  for (int l = 0; l < 9; ++l) gm[l] = 0.5 * (__ldg(met + ida + l * sz) + __ldg(met + idb + l * sz));
+  for (int l = 0; l < 9; ++l) gm[l] = 0.5 * (ma[l] + mb[l]);
   double dd[4][3];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -300,10 +299,9 @@ __device__ __forceinline__ void ring_face(const RingSmem &S, const double *__res
   const double tau_xy = mul * (u_y + v_x);
   const double tau_xz = mul * (u_z + w_x);
   const double tau_yz = mul * (v_z + w_y);
-  const double ja = __ldg(jac + ida), jb = __ldg(jac + idb);
-  const double gk0 = 0.5 * (__ldg(met + ida + (3 * DIR) * sz) * ja + __ldg(met + idb + (3 * DIR) * sz) * jb);
-  const double gk1 = 0.5 * (__ldg(met + ida + (3 * DIR + 1) * sz) * ja + __ldg(met + idb + (3 * DIR + 1) * sz) * jb);
-  const double gk2 = 0.5 * (__ldg(met + ida + (3 * DIR + 2) * sz) * ja + __ldg(met + idb + (3 * DIR + 2) * sz) * jb);
+  const double gk0 = 0.5 * (ma[3 * DIR] * ma[9] + mb[3 * DIR] * mb[9]);
+  const double gk1 = 0.5 * (ma[3 * DIR + 1] * ma[9] + mb[3 * DIR + 1] * mb[9]);
+  const double gk2 = 0.5 * (ma[3 * DIR + 2] * ma[9] + mb[3 * DIR + 2] * mb[9]);
   F[0] = gk0 * tau_xx + gk1 * tau_xy + gk2 * tau_xz;
   F[1] = gk0 * tau_xy + gk1 * tau_yy + gk2 * tau_yz;
   F[2] = gk0 * tau_xz + gk1 * tau_yz + gk2 * tau_zz;
@@ -315,13 +313,19 @@ __device__ __forceinline__ void ring_face(const RingSmem &S, const double *__res
 }
 }  // namespace
 
-// MINB: CTAs per SM the register budget is sized for (2: no spills; 3: about
-// 80 registers with a few spills, 24 warps per SM).  PF: with the request of
-// plane k+2's dynamic values, also ask L2 for its metric and J (the faces of
-// plane k+2 read them through L1 two planes later), so that those loads no
-// longer wait on DRAM.
+// MINB: CTAs per SM the register budget is sized for.  PF: with the request of
+// plane k+2's dynamic values, also ask L2 for its metric and J, so that the
+// faces' reads of them no longer wait on DRAM.
+//
+// Bound by the L1 and shared-memory pipe and by the barriers of a plane.  A
+// thread holds its node's metric and J in registers for its lower x and y faces
+// and both its z faces and reads its neighbours' once (30 loads a plane instead
+// of some 60).  145 x 130 x 99 (us): faces shared out with every metric read
+// from L1 234; the same 32 x 8 tile with the metric held 212; 32 x 4, 128
+// threads, four CTAs of 128 registers 180, three of 158 registers 181, which is
+// the faster on large blocks (257^3 step 29.02, 28.68 ms).
 template <int MINB, bool PF>
-__global__ void __launch_bounds__(kFT, MINB) viscous_air_ring(Zone z, double Pr) {
+__global__ void __launch_bounds__(kFT, MINB) viscous_air_ring(Zone z, double Pr, int planes) {
   extern __shared__ __align__(16) double rsm[];
   const double cp_pr = kCpAir / Pr;
   RingSmem &S = *reinterpret_cast<RingSmem *>(rsm);
@@ -329,10 +333,10 @@ __global__ void __launch_bounds__(kFT, MINB) viscous_air_ring(Zone z, double Pr)
   const int g = d.ngg;
   const int64_t sz = d.plane(g), szq = d.plane(0);
   const int64_t srow = d.stride(g, 1), spl = d.stride(g, 2);
-  const int i0 = blockIdx.x * kFX, j0 = blockIdx.y * kFY, k0 = blockIdx.z * kFZ;
+  const int i0 = blockIdx.x * kFX, j0 = blockIdx.y * kFY, k0 = blockIdx.z * planes;
   const int tx = threadIdx.x % kFX, ty = threadIdx.x / kFX;
   const bool three_d = d.mz > 1;
-  const int k_end = min(k0 + kFZ, d.mz);
+  const int k_end = min(k0 + planes, d.mz);
   const double *__restrict__ met = z.metric;
   const double *__restrict__ jac = z.jac;
 
@@ -359,26 +363,34 @@ __global__ void __launch_bounds__(kFT, MINB) viscous_air_ring(Zone z, double Pr)
   request(k0, 1);
   request(k0 + 1, 2);
   cp_async_commit();
-  cp_async_wait_all();
-  __syncthreads();
   const int i = i0 + tx, j = j0 + ty;
   const bool mine = i < d.mx && j < d.my;
+  // the lower x and y faces of the node, also where it is the first beyond the block
+  const bool face_x = i <= d.mx && j < d.my, face_y = i < d.mx && j <= d.my;
+  auto load_m = [&](int64_t id, double (&m)[10]) {
+#pragma unroll
+    for (int l = 0; l < 9; ++l) m[l] = __ldg(met + id + l * sz);
+    m[9] = __ldg(jac + id);
+  };
+  // metric and J of this thread's node on plane k: read once, used by its
+  // three faces and by the z face of the next plane
+  double mc[10];
+  const int64_t id0 = d.idx(g, min(i, d.mx), min(j, d.my), k0);
+  load_m(id0, mc);
+  cp_async_wait_all();
+  __syncthreads();
   double fzp[4] = {0, 0, 0, 0};
   if (three_d && mine) {
-    const int64_t ida = d.idx(g, i, j, k0 - 1);
-    ring_face<2>(S, met, jac, sz, 0, tx + 1, ty + 1, ida, 1, tx + 1, ty + 1, ida + spl, cp_pr, fzp);
+    double mb[10];
+    load_m(id0 - spl, mb);
+    ring_face<2>(S, 0, tx + 1, ty + 1, mb, 1, tx + 1, ty + 1, mc, cp_pr, fzp);
   }
   // the first iteration refills slot 0, which the z faces above read at
   // neighbouring points
   __syncthreads();
   int sp = 0, sc = 1, sn = 2;  // slots of planes k-1, k, k+1
   for (int k = k0; k < k_end; ++k) {
-    double acc[4];
-    const int64_t iq = d.idx(0, i, j, k);
-    if (mine) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] = z.dq[iq + (q + 1) * szq];
-    }
+    const int64_t id = id0 + (k - k0) * spl;
     // k-differences at this thread's points: its own copies of planes k-1
     // and k+1 are complete, and no other thread reads these points of
     // slot sp before the next barrier
@@ -390,57 +402,69 @@ __global__ void __launch_bounds__(kFT, MINB) viscous_air_ring(Zone z, double Pr)
       for (int q = 0; q < 4; ++q) S.dzp[q][py][px] = S.dyn[sn][q][py][px] - S.dyn[sp][q][py][px];
     }
     if (k + 2 <= k_end) request(k + 2, sp);  // plane k+2 into the slot of plane k-1
-    if (PF && k + 2 <= k_end) {
+    if (PF && k + 2 <= k_end && face_x) {
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        int px, py;
-        if (!point_ok(threadIdx.x + r * kFT, px, py)) continue;
-        const int64_t id = d.idx(g, i0 - 1 + px, j0 - 1 + py, k + 2);
-#pragma unroll
-        for (int m = 0; m < 9; ++m) prefetch_l2(met + id + m * sz);
-        prefetch_l2(jac + id);
-      }
+      for (int m = 0; m < 9; ++m) prefetch_l2(met + id + 2 * spl + m * sz);
+      prefetch_l2(jac + id + 2 * spl);
     }
     cp_async_commit();
     __syncthreads();
-    constexpr int kNXF = kFY * (kFX + 1), kNYF = (kFY + 1) * kFX;
-    constexpr int kYF0 = (kNXF + 31) / 32 * 32;
-    for (int f = threadIdx.x; f < kYF0 + kNYF; f += kFT) {
-      if (f < kYF0) {
-        if (f >= kNXF) continue;
-        const int fy_ = f / (kFX + 1), fx_ = f - fy_ * (kFX + 1);
-        if (i0 - 1 + fx_ > d.mx - 1 || j0 + fy_ >= d.my) continue;
-        const int64_t ida = d.idx(g, i0 - 1 + fx_, j0 + fy_, k);
-        double F[4];
-        ring_face<0>(S, met, jac, sz, sc, fx_, fy_ + 1, ida, sc, fx_ + 1, fy_ + 1, ida + 1, cp_pr, F);
+    double fx[4], fy[4];
+    if (face_x) {
+      double ma[10];
+      load_m(id - 1, ma);
+      ring_face<0>(S, sc, tx, ty + 1, ma, sc, tx + 1, ty + 1, mc, cp_pr, fx);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) S.fx[q][fy_][fx_] = F[q];
-      } else {
-        const int e = f - kYF0;
-        const int fy_ = e / kFX, fx_ = e - fy_ * kFX;
-        if (i0 + fx_ >= d.mx || j0 - 1 + fy_ > d.my - 1) continue;
-        const int64_t ida = d.idx(g, i0 + fx_, j0 - 1 + fy_, k);
-        double F[4];
-        ring_face<1>(S, met, jac, sz, sc, fx_ + 1, fy_, ida, sc, fx_ + 1, fy_ + 1, ida + srow, cp_pr, F);
+      for (int q = 0; q < 4; ++q) S.fx[q][ty][tx] = fx[q];
+    }
+    if (face_y) {
+      double ma[10];
+      load_m(id - srow, ma);
+      ring_face<1>(S, sc, tx + 1, ty, ma, sc, tx + 1, ty + 1, mc, cp_pr, fy);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) S.fy[q][fy_][fx_] = F[q];
+      for (int q = 0; q < 4; ++q) S.fy[q][ty][tx] = fy[q];
+    }
+    // the tile's last y faces and last x faces: a warp each, another one on every plane
+    if (ty == (k & (kFY - 1))) {
+      if (i < d.mx && j0 + kFY <= d.my) {
+        double ma[10], mb[10], F[4];
+        const int64_t ida = d.idx(g, i, j0 + kFY - 1, k);
+        load_m(ida, ma);
+        load_m(ida + srow, mb);
+        ring_face<1>(S, sc, tx + 1, kFY, ma, sc, tx + 1, kFY + 1, mb, cp_pr, F);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) S.fy[q][kFY][tx] = F[q];
+      }
+    } else if (ty == ((k + kFY / 2) & (kFY - 1)) && tx < kFY) {
+      if (j0 + tx < d.my && i0 + kFX <= d.mx) {
+        double ma[10], mb[10], F[4];
+        const int64_t ida = d.idx(g, i0 + kFX - 1, j0 + tx, k);
+        load_m(ida, ma);
+        load_m(ida + 1, mb);
+        ring_face<0>(S, sc, kFX, tx + 1, ma, sc, kFX + 1, tx + 1, mb, cp_pr, F);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) S.fx[q][tx][kFX] = F[q];
       }
     }
     double fzn[4] = {0, 0, 0, 0};
-    if (three_d && mine) {
-      const int64_t ida = d.idx(g, i, j, k);
-      ring_face<2>(S, met, jac, sz, sc, tx + 1, ty + 1, ida, sn, tx + 1, ty + 1, ida + spl, cp_pr, fzn);
+    if (three_d) {
+      double mn[10];
+      load_m(id + spl, mn);
+      if (mine) ring_face<2>(S, sc, tx + 1, ty + 1, mc, sn, tx + 1, ty + 1, mn, cp_pr, fzn);
+#pragma unroll
+      for (int l = 0; l < 10; ++l) mc[l] = mn[l];
     }
     cp_async_wait_all();
     __syncthreads();
     if (mine) {
+      // the differences in x, y, z order; one addition to dq
+      const int64_t iq = d.idx(0, i, j, k);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        double a = acc[q];
-        a += S.fx[q][ty][tx + 1] - S.fx[q][ty][tx];
-        a += S.fy[q][ty + 1][tx] - S.fy[q][ty][tx];
+        double a = S.fx[q][ty][tx + 1] - fx[q];
+        a += S.fy[q][ty + 1][tx] - fy[q];
         if (three_d) a += fzn[q] - fzp[q];
-        z.dq[iq + (q + 1) * szq] = a;
+        red_add(z.dq + iq + (q + 1) * szq, a);
       }
     }
 #pragma unroll
@@ -452,16 +476,36 @@ __global__ void __launch_bounds__(kFT, MINB) viscous_air_ring(Zone z, double Pr)
   }
 }
 
-// Opt the kernel in to its dynamic shared-memory size (108 KB, two CTAs per SM).
+// Opt the kernels in to their dynamic shared-memory sizes.
 cudaError_t viscous_air_init_attributes() {
   cudaError_t e = cudaFuncSetAttribute(viscous_air_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)sizeof(FusedSmem));
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(viscous_air_ring<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  e = cudaFuncSetAttribute(viscous_air_ring<kCtas, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)sizeof(RingSmem));
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(viscous_air_ring<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(viscous_air_ring<kCtas, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)sizeof(RingSmem));
+}
+
+// Planes a CTA marches through: of all equal cuts of the block along k, the one
+// with the fewest plane steps in its last CTA to finish, waves of kCtas CTAs
+// an SM times a chunk's planes and the two that its start costs.  With 32 planes
+// always, small blocks were a handful of CTAs (us: 40 x 37 x 33 137, 22 with the
+// chunks cut to fit; 64 x 257 x 20 96, 45; 90 x 80 x 70 150, 66).
+int viscous_chunk(long long tiles, int mz, int n_sm) {
+  long long best = -1;
+  int planes = mz;
+  for (int c = 1; c <= mz; ++c) {
+    const int len = (mz + c - 1) / c;
+    if (c > 1 && len == (mz + c - 2) / (c - 1)) continue;  // the same chunks with an empty one
+    const long long cost = (tiles * c + (long long)kCtas * n_sm - 1) / ((long long)kCtas * n_sm) * (len + 2);
+    if (best < 0 || cost < best) {
+      best = cost;
+      planes = len;
+    }
+  }
+  return planes;
 }
 
 // compute_viscous_flux for air (reference src/ViscousScheme.cu:7-40): one
@@ -469,10 +513,12 @@ cudaError_t viscous_air_init_attributes() {
 // 2 the ring kernel with the L2 prefetch of the metric two planes ahead.
 cudaError_t launch_viscous_air(const Zone &z, const Param &p, cudaStream_t st, int *n_launch, int var) {
   const Dims &d = z.d;
-  const dim3 grid((d.mx + kFX - 1) / kFX, (d.my + kFY - 1) / kFY, (d.mz + kFZ - 1) / kFZ);
-  if (var == 1) viscous_air_ring<2, false><<<grid, kFT, sizeof(RingSmem), st>>>(z, p.Pr);
-  else if (var == 2) viscous_air_ring<2, true><<<grid, kFT, sizeof(RingSmem), st>>>(z, p.Pr);
-  else viscous_air_fused<<<grid, kFT, sizeof(FusedSmem), st>>>(z, p.Pr);
+  dim3 grid((d.mx + kFX - 1) / kFX, (d.my + kFY - 1) / kFY);
+  const int planes = viscous_chunk((long long)grid.x * grid.y, d.mz, 148);
+  grid.z = (d.mz + planes - 1) / planes;
+  if (var == 1) viscous_air_ring<kCtas, false><<<grid, kFT, sizeof(RingSmem), st>>>(z, p.Pr, planes);
+  else if (var == 2) viscous_air_ring<kCtas, true><<<grid, kFT, sizeof(RingSmem), st>>>(z, p.Pr, planes);
+  else viscous_air_fused<<<grid, kFT, sizeof(FusedSmem), st>>>(z, p.Pr, planes);
   *n_launch += 1;
   return cudaGetLastError();
 }

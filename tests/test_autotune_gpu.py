@@ -159,3 +159,21 @@ def test_untuned_air_tiles_by_block_size(scheme, n, ny, nz):
         oz.initialize()
         oz.call("orc_compute_inviscid_flux")
         assert rel_err(out[0], oz["dq"]) <= 1e-11
+
+
+@pytest.mark.parametrize("n, ny, nz", [(31, 4, 7), (32, 5, 9), (33, 8, 40), (64, 9, 5), (95, 36, 33)])
+def test_viscous_forms_at_tile_and_chunk_edges(n, ny, nz):
+    """Every form of the air viscous kernel on extents at the edges of its 32 x
+    4 tiles and of its chunks of planes, against the oracle (1e-11, single
+    call)."""
+    case = cases.perturbed(cases.sine_wave(n=n, ny=ny, nz=nz, scheme=2, viscous=True), seed=5, amp=1e-2)
+    oz = pyoracle.OracleZone(case)
+    oz.initialize()
+    oz.call("orc_compute_viscous_flux")
+    gz = GpuZone(case)
+    gz.initialize()
+    for form in (0, 1, 2):
+        gz.t["dq"].zero_()
+        gz.ctx.viscous_variant(form)
+        gz.ctx.viscous()
+        assert rel_err(gz.get("dq"), oz["dq"]) <= 1e-11, form
