@@ -585,6 +585,131 @@ __global__ void sg_colstats_kernel(const float *X, const float *G, long long n, 
 }
 
 // ---------------------------------------------------------------------------
+// Inference over a table of raw features
+// ---------------------------------------------------------------------------
+// Forward pass of n rows.  Three 128-thread groups a CTA, one CTA an SM, each
+// group on its own 128-row tiles with its own operand tiles and TMEM columns:
+// while one group waits for its GEMM the others are in their tanh epilogues,
+// which bound the kernel (384 a row at 16 a clock and SM).  With one tile in
+// flight an SM a tile took 11 700 cycles.  The next tile's features are read
+// during the current one's GEMMs.
+constexpr int kFwdGroups = 3;
+constexpr int kFwdMbar = kSgWBytes + kFwdGroups * kStepGroup;
+constexpr int kFwdSmem = kFwdMbar + 64;
+static_assert(kFwdSmem <= 227 * 1024, "forward kernel shared memory");
+
+struct SgForwardArgs {
+  const float *X;
+  float *Y;  // [n][16] standardised outputs
+  int n;
+  int vec;   // X and Y are 16-byte aligned
+  SgNorm nrm;
+  const uint8_t *w16;
+  int *err;
+};
+
+__global__ void __launch_bounds__(128 * kFwdGroups, 1) sg_forward_kernel(const __grid_constant__ SgForwardArgs a) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, g = warp >> 2, row = tid & 127;
+  uint8_t *sa0 = smem + kSgWBytes + g * kStepGroup, *sact = sa0 + kTileA0;
+  uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kFwdMbar);
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + kFwdMbar + 8 * kFwdGroups);
+#pragma unroll 8
+  for (int o = tid * 16; o < kSgWBytes; o += 128 * kFwdGroups * 16)
+    *reinterpret_cast<uint4 *>(smem + o) = __ldg(reinterpret_cast<const uint4 *>(a.w16 + o));
+  init_const_cols(sact, row);
+  if (tid == 0) {
+    for (int q = 0; q < kFwdGroups; ++q) mbar_init(smem_addr(&mbar[q]), 1);
+    mbar_init_fence();
+  }
+  if (warp == 0) tmem_alloc(smem_addr(tslot), 512);
+  fence_proxy_async();
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tb = *tslot, tcol = tb + g * 128;
+  const uint32_t tl = tcol + ((uint32_t)(32 * (warp & 3)) << 16);
+  const uint32_t mb = smem_addr(&mbar[g]), a0s = smem_addr(sa0), acts = smem_addr(sact), ws = smem_addr(smem);
+  const int bar_id = 1 + g;
+  const uint32_t id_h = idesc_bf16(128, 128, 0, 0), id_o = idesc_bf16(128, 16, 0, 0);
+  uint32_t phase = 0;
+  bool bad = false;
+
+  auto run = [&](int layer) -> bool {
+    fence_proxy_async();
+    fence_before_sync();
+    group_bar(bar_id);
+    if (row == 0) {
+      fence_after_sync();
+      if (layer == 0) gemm(tcol, a0s, 16, false, ws + 2 * kSgW0, 16, false, 1, id_h, false);
+      else if (layer == 1) gemm(tcol, acts, 144, false, ws + 2 * kSgW1, 144, false, 9, id_h, false);
+      else if (layer == 2) gemm(tcol, acts, 144, false, ws + 2 * kSgW2, 144, false, 9, id_h, false);
+      else gemm(tcol, acts, 144, false, ws + 2 * kSgW3, 144, false, 9, id_o, false);
+      mma_commit(mb);
+    }
+    const bool ok = mbar_wait(mb, phase, kWaitCycles);
+    phase ^= 1u;
+    const bool any_bad = group_any(bar_id, !ok);
+    fence_after_sync();
+    return !any_bad;
+  };
+  auto load_x = [&](int r, float (&x)[kSgIn]) {
+    if (r >= a.n) {
+      for (int c = 0; c < kSgIn; ++c) x[c] = a.nrm.in_mean[c];
+    } else if (a.vec) {
+      const float4 *p = reinterpret_cast<const float4 *>(a.X + (long long)r * kSgIn);
+#pragma unroll
+      for (int c = 0; c < kSgIn / 4; ++c) {
+        const float4 v = __ldg(p + c);
+        x[4 * c] = v.x; x[4 * c + 1] = v.y; x[4 * c + 2] = v.z; x[4 * c + 3] = v.w;
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < kSgIn; ++c) x[c] = __ldg(a.X + (long long)r * kSgIn + c);
+    }
+  };
+
+  const int n_tiles = (int)(((long long)a.n + 127) / 128), step = gridDim.x * kFwdGroups;
+  float x[kSgIn];
+  int t = blockIdx.x + g * gridDim.x;  // a CTA's groups share the work of small tables
+  if (t < n_tiles) load_x(t * 128 + row, x);
+  for (; t < n_tiles; t += step) {
+    const int r = t * 128 + row;
+    const bool valid = r < a.n;
+#pragma unroll
+    for (int c = 0; c < kSgIn; ++c) x[c] = (x[c] - a.nrm.in_mean[c]) * a.nrm.in_rstd[c];
+    write_a0_row(sa0, row, x, valid ? 1.f : 0.f);
+    if (t + step < n_tiles) load_x(r + step * 128, x);
+    if (!run(0)) { bad = true; break; }
+    epi_tanh(tl, sact, row);
+    if (!run(1)) { bad = true; break; }
+    epi_tanh(tl, sact, row);
+    if (!run(2)) { bad = true; break; }
+    epi_tanh(tl, sact, row);
+    if (!run(3)) { bad = true; break; }
+    float y[16];
+    tmem_ld16(tl, y);
+    if (!valid) continue;
+    float *o = a.Y + (long long)r * 16;
+    if (a.vec) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        reinterpret_cast<float4 *>(o)[c] = make_float4(y[4 * c], y[4 * c + 1], y[4 * c + 2], y[4 * c + 3]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 16; ++c) o[c] = y[c];
+    }
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    fence_after_sync();
+    tmem_dealloc(tb, 512);
+  }
+  if (bad && row == 0) atomicOr(a.err, 4);
+}
+
+// ---------------------------------------------------------------------------
 // Training: fused forward + backward of one minibatch
 // ---------------------------------------------------------------------------
 struct SgTrainArgs {
@@ -593,12 +718,10 @@ struct SgTrainArgs {
   long long perm_a, perm_b;  // row of minibatch entry i: (perm_a * i + perm_b) mod n
   long long start;           // first minibatch entry
   int count;                 // minibatch rows
-  int mode;                  // 0: gradients, 1: forward outputs only
   SgNorm nrm;
   const uint8_t *w16;
   float *partials;           // [gridDim.x][kSgNParam]
   double *loss;
-  float *Yout;               // mode 1: [n][16] standardised outputs
   int *err;
 };
 
@@ -611,6 +734,7 @@ __global__ void __launch_bounds__(128, 1) sg_train_kernel(const __grid_constant_
   uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kTrMbar);
   uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + kTrMbar + 8);
 
+#pragma unroll 8
   for (int o = tid * 16; o < kSgWBytes; o += 128 * 16)
     *reinterpret_cast<uint4 *>(sw + o) = __ldg(reinterpret_cast<const uint4 *>(a.w16 + o));
   init_const_cols(sh1, row);
@@ -687,7 +811,6 @@ __global__ void __launch_bounds__(128, 1) sg_train_kernel(const __grid_constant_
       s = (long long)(((unsigned long long)a.perm_a * (unsigned long long)(a.start + r) + (unsigned long long)a.perm_b) %
                       (unsigned long long)a.n);
       for (int c = 0; c < kSgIn; ++c) x[c] = (a.X[s * kSgIn + c] - a.nrm.in_mean[c]) * a.nrm.in_rstd[c];
-      if (a.mode == 0)
         for (int c = 0; c < kSgOut; ++c) {
           const float g = a.G[s * kSgOut + c], sc = a.nrm.out_scale[c];
           tgt[c] = ((sc > 0.f ? asinhf(g / sc) : g) - a.nrm.out_mean[c]) / a.nrm.out_std[c];
@@ -706,11 +829,6 @@ __global__ void __launch_bounds__(128, 1) sg_train_kernel(const __grid_constant_
     if (!run(3)) { bad = true; break; }
     float y[16];
     tmem_ld16(tsc + lane_off, y);
-    if (a.mode == 1) {
-      if (valid)
-        for (int c = 0; c < 16; ++c) a.Yout[s * 16 + c] = y[c];
-      continue;
-    }
     float dy[16];
     for (int c = 0; c < 16; ++c) {
       const float e = (valid && c < kSgOut) ? y[c] - tgt[c] : 0.f;
@@ -737,7 +855,10 @@ __global__ void __launch_bounds__(128, 1) sg_train_kernel(const __grid_constant_
     first = false;
   }
 
-  if (a.mode == 0 && !bad) {
+  if (!bad) {
+    // the blocks of 128 rows by columns, so that a warp's lanes (rows) write
+    // 128 consecutive bytes: row by row the stores of a CTA's 165 KB took half
+    // of the kernel
     float *part = a.partials + (long long)blockIdx.x * kSgNParam;
     const int o = row;  // TMEM lane = output row (dW0, dW1, dW2) or input row (dW3^T)
     if (first) {
@@ -747,16 +868,16 @@ __global__ void __launch_bounds__(128, 1) sg_train_kernel(const __grid_constant_
       float v[32];
       for (int cb = 0; cb < 4; ++cb) {
         tmem_ld32(tb + kTmDW1 + lane_off + cb * 32, v);
-        for (int c = 0; c < 32; ++c) part[kSgW1 + o * 144 + cb * 32 + c] = v[c];
+        for (int c = 0; c < 32; ++c) part[kSgW1 + (cb * 32 + c) * 128 + o] = v[c];
         tmem_ld32(tb + kTmDW2 + lane_off + cb * 32, v);
-        for (int c = 0; c < 32; ++c) part[kSgW2 + o * 144 + cb * 32 + c] = v[c];
+        for (int c = 0; c < 32; ++c) part[kSgW2 + (cb * 32 + c) * 128 + o] = v[c];
       }
       tmem_ld16(tb + kTmDW1 + lane_off + 128, v);
-      for (int c = 0; c < 16; ++c) part[kSgW1 + o * 144 + 128 + c] = v[c];
+      for (int c = 0; c < 16; ++c) part[kSgW1 + (128 + c) * 128 + o] = v[c];
       tmem_ld16(tb + kTmDW2 + lane_off + 128, v);
-      for (int c = 0; c < 16; ++c) part[kSgW2 + o * 144 + 128 + c] = v[c];
+      for (int c = 0; c < 16; ++c) part[kSgW2 + (128 + c) * 128 + o] = v[c];
       tmem_ld16(tb + kTmDW0 + lane_off, v);
-      for (int c = 0; c < 16; ++c) part[kSgW0 + o * 16 + c] = v[c];
+      for (int c = 0; c < 16; ++c) part[kSgW0 + c * 128 + o] = v[c];
       tmem_ld16(tb + kTmDW3 + lane_off, v);
       for (int c = 0; c < 16; ++c) part[kSgW3 + c * 144 + o] = v[c];
       __syncthreads();
@@ -766,7 +887,7 @@ __global__ void __launch_bounds__(128, 1) sg_train_kernel(const __grid_constant_
       }
     }
   }
-  if (a.mode == 0) {
+  {
     double l = loss_acc;
     for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
     if (lane == 0) atomicAdd(a.loss, l);
@@ -787,11 +908,19 @@ __global__ void __launch_bounds__(128, 1) sg_train_kernel(const __grid_constant_
 // until the host reads the flag and reports the error.
 __global__ void sg_adam_kernel(float *master, float *m, float *v, const float *partials, int n_part, uint8_t *w16,
                                float lr, float b1, float b2, float eps, float bc1, float bc2, float *grad_out,
-                               int update, const int *err) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= kSgNParam) return;
+                               int update, const int *err, double *status) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (status && t == 0) *status = (double)*(volatile const int *)err;  // read back with the loss
+  if (t >= kSgNParam) return;
+  // partials hold the blocks of 128 rows by columns (sg_train_kernel)
+  int e = t;
+  if (t < kSgW3) {
+    const int base = t < kSgW1 ? kSgW0 : t < kSgW2 ? kSgW1 : kSgW2, q = t - base;
+    e = base + (q & 127) * (t < kSgW1 ? 16 : 144) + (q >> 7);
+  }
   float g = 0.f;
-  for (int p = 0; p < n_part; ++p) g += partials[(long long)p * kSgNParam + e];
+#pragma unroll 8
+  for (int p = 0; p < n_part; ++p) g += partials[(long long)p * kSgNParam + t];
   if (grad_out) grad_out[e] = g;
   if (!update) return;
   if (err && (*(volatile const int *)err & 4)) return;
@@ -835,6 +964,8 @@ __global__ void sg_init_kernel(float *master, float *m, float *v, unsigned long 
 // ---------------------------------------------------------------------------
 cudaError_t sg_init_attributes() {
   cudaError_t e = cudaFuncSetAttribute(sg_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(sg_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(sg_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem);
 }
@@ -885,14 +1016,24 @@ cudaError_t launch_sg_colstats(const float *X, const float *G, long long n, cons
   return cudaGetLastError();
 }
 
+cudaError_t launch_sg_forward(const float *X, int n, const SgNorm &nrm, const uint8_t *w16, float *Y, int *err,
+                              int n_sm, cudaStream_t st) {
+  SgForwardArgs a;
+  a.X = X; a.Y = Y; a.n = n; a.nrm = nrm; a.w16 = w16; a.err = err;
+  a.vec = ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15) == 0;
+  const long long tiles = ((long long)n + 127) / 128;
+  const int grid = (int)(tiles < n_sm ? tiles : n_sm);
+  sg_forward_kernel<<<grid, 128 * kFwdGroups, kFwdSmem, st>>>(a);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_sg_train(const float *X, const float *G, long long n, long long perm_a, long long perm_b,
-                            long long start, int count, int mode, const SgNorm &nrm, const uint8_t *w16,
-                            float *partials, int max_ctas, double *loss, float *Yout, int *err, int *n_ctas,
-                            cudaStream_t st) {
+                            long long start, int count, const SgNorm &nrm, const uint8_t *w16, float *partials,
+                            int max_ctas, double *loss, int *err, int *n_ctas, cudaStream_t st) {
   SgTrainArgs a;
-  a.X = X; a.G = G; a.n = n; a.perm_a = perm_a; a.perm_b = perm_b; a.start = start; a.count = count; a.mode = mode;
-  a.nrm = nrm; a.w16 = w16; a.partials = partials; a.loss = loss; a.Yout = Yout; a.err = err;
-  int grid = (count + 127) / 128;
+  a.X = X; a.G = G; a.n = n; a.perm_a = perm_a; a.perm_b = perm_b; a.start = start; a.count = count;
+  a.nrm = nrm; a.w16 = w16; a.partials = partials; a.loss = loss; a.err = err;
+  int grid = (int)(((long long)count + 127) / 128);
   if (grid > max_ctas) grid = max_ctas;
   if (grid < 1) grid = 1;
   *n_ctas = grid;
@@ -902,9 +1043,9 @@ cudaError_t launch_sg_train(const float *X, const float *G, long long n, long lo
 
 cudaError_t launch_sg_adam(float *master, float *m, float *v, const float *partials, int n_part, uint8_t *w16,
                            float lr, float b1, float b2, float eps, float bc1, float bc2, float *grad_out, int update,
-                           const int *err, cudaStream_t st) {
-  sg_adam_kernel<<<(kSgNParam + 255) / 256, 256, 0, st>>>(master, m, v, partials, n_part, w16, lr, b1, b2, eps, bc1,
-                                                          bc2, grad_out, update, err);
+                           const int *err, double *status, cudaStream_t st) {
+  sg_adam_kernel<<<(kSgNParam + 127) / 128, 128, 0, st>>>(master, m, v, partials, n_part, w16, lr, b1, b2, eps, bc1,
+                                                          bc2, grad_out, update, err, status);
   return cudaGetLastError();
 }
 

@@ -24,13 +24,14 @@ cudaError_t launch_sg_snapshot(const Zone &z, const Thermo *th, double dt, doubl
 cudaError_t launch_sg_record(const Zone &z, int ns, const double *snap, double dt, float *X, float *G, cudaStream_t st);
 cudaError_t launch_sg_colstats(const float *X, const float *G, long long n, const float *scales, double *acc,
                                unsigned *mm, int n_sm, cudaStream_t st);
+cudaError_t launch_sg_forward(const float *X, int n, const SgNorm &nrm, const uint8_t *w16, float *Y, int *err,
+                              int n_sm, cudaStream_t st);
 cudaError_t launch_sg_train(const float *X, const float *G, long long n, long long perm_a, long long perm_b,
-                            long long start, int count, int mode, const SgNorm &nrm, const uint8_t *w16,
-                            float *partials, int max_ctas, double *loss, float *Yout, int *err, int *n_ctas,
-                            cudaStream_t st);
+                            long long start, int count, const SgNorm &nrm, const uint8_t *w16, float *partials,
+                            int max_ctas, double *loss, int *err, int *n_ctas, cudaStream_t st);
 cudaError_t launch_sg_adam(float *master, float *m, float *v, const float *partials, int n_part, uint8_t *w16,
                            float lr, float b1, float b2, float eps, float bc1, float bc2, float *grad_out, int update,
-                           const int *err, cudaStream_t st);
+                           const int *err, double *status, cudaStream_t st);
 cudaError_t launch_sg_publish(const float *master, uint8_t *w16, cudaStream_t st);
 cudaError_t launch_sg_init(float *master, float *m, float *v, unsigned long long seed, cudaStream_t st);
 cudaError_t launch_wu_reaction_list(const Zone &z, const Param &p, const Mech *mc, const Mech &mc_host, double dt,
@@ -261,14 +262,14 @@ int cfk_surrogate_train(cfk_ctx *c, const float *X, const float *G, long long n,
     for (long long st = 0; st < n; st += batch, ++step) {
       const int count = (int)std::min<long long>(batch, n - st);
       int n_ctas = 0;
-      CFK_CHECK(c, launch_sg_train(X, G, n, pa, pb, st, count, 0, s->norm, s->w16, s->partials, c->n_sm, s->loss,
-                                   nullptr, c->d_err, &n_ctas, 0),
+      CFK_CHECK(c, launch_sg_train(X, G, n, pa, pb, st, count, s->norm, s->w16, s->partials, c->n_sm, s->loss,
+                                   c->d_err, &n_ctas, 0),
                 "surrogate train");
       const double lr = lr1 + 0.5 * (lr0 - lr1) * (1.0 + std::cos(M_PI * (double)step / (double)total));
       s->adam_t += 1;
       const float bc1 = 1.f - std::pow(b1, (float)s->adam_t), bc2 = 1.f - std::pow(b2, (float)s->adam_t);
       CFK_CHECK(c, launch_sg_adam(s->master, s->m, s->v, s->partials, n_ctas, s->w16, (float)lr, b1, b2, eps, bc1,
-                                  bc2, nullptr, 1, c->d_err, 0),
+                                  bc2, nullptr, 1, c->d_err, nullptr, 0),
                 "surrogate adam");
       c->launches += 2;
     }
@@ -291,20 +292,18 @@ int cfk_surrogate_gradients(cfk_ctx *c, const float *X, const float *G, long lon
   Surrogate *s = c->sg;
   CFK_CHECK(c, cudaMemset(s->loss, 0, sizeof(double)), "loss reset");
   int n_ctas = 0;
-  CFK_CHECK(c, launch_sg_train(X, G, n, 1, 0, 0, (int)n, 0, s->norm, s->w16, s->partials, c->n_sm, s->loss, nullptr,
-                               c->d_err, &n_ctas, 0),
+  CFK_CHECK(c, launch_sg_train(X, G, n, 1, 0, 0, (int)n, s->norm, s->w16, s->partials, c->n_sm, s->loss, c->d_err,
+                               &n_ctas, 0),
             "surrogate gradients");
   CFK_CHECK(c, launch_sg_adam(s->master, s->m, s->v, s->partials, n_ctas, s->w16, 0.f, 0.9f, 0.999f, 1e-8f, 1.f, 1.f,
-                              grad_out, 0, nullptr, 0),
+                              grad_out, 0, c->d_err, s->loss + 1, 0),
             "gradient reduction");
   c->launches += 2;
-  CFK_CHECK(c, cudaDeviceSynchronize(), "surrogate gradients");
-  if (loss_out) {
-    double l = 0;
-    CFK_CHECK(c, cudaMemcpy(&l, s->loss, sizeof(double), cudaMemcpyDeviceToHost), "loss read");
-    *loss_out = l / ((double)n * kSgOut);
-  }
-  return check_err_flags(c);
+  // one read back: the loss and, beside it, the error flag; it waits for the kernels
+  double back[2] = {0, 0};
+  CFK_CHECK(c, cudaMemcpy(back, s->loss, sizeof(back), cudaMemcpyDeviceToHost), "loss read");
+  if (loss_out) *loss_out = back[0] / ((double)n * kSgOut);
+  return ((int)back[1] & 4) ? check_err_flags(c) : CFK_OK;
 }
 
 int cfk_surrogate_forward(cfk_ctx *c, const float *X, long long n, float *Y) {
@@ -314,13 +313,9 @@ int cfk_surrogate_forward(cfk_ctx *c, const float *X, long long n, float *Y) {
   if (!X || !Y || n < 1 || n > 2147483647LL) return fail(c, CFK_ERR_ARG, "bad forward arguments");
   CFK_CHECK(c, cudaSetDevice(c->hp.device), "cudaSetDevice");
   Surrogate *s = c->sg;
-  int n_ctas = 0;
-  CFK_CHECK(c, launch_sg_train(X, X, n, 1, 0, 0, (int)n, 1, s->norm, s->w16, s->partials, c->n_sm, s->loss, Y,
-                               c->d_err, &n_ctas, 0),
-            "surrogate forward");
+  CFK_CHECK(c, launch_sg_forward(X, (int)n, s->norm, s->w16, Y, c->d_err, c->n_sm, 0), "surrogate forward");
   c->launches += 1;
-  CFK_CHECK(c, cudaDeviceSynchronize(), "surrogate forward");
-  return check_err_flags(c);
+  return check_err_flags(c);  // its read back waits for the kernel
 }
 
 int cfk_surrogate_get_params(cfk_ctx *c, float *weights, float *norm) {

@@ -261,3 +261,32 @@ def test_trained_surrogate_throughput_on_burnt_mix(trained):
     print(f"plain {ms['plain']:.1f} ms, surrogate {ms['surrogate']:.1f} ms, "
           f"speed-up {ms['plain'] / ms['surrogate']:.2f}x")
     assert ms["plain"] / ms["surrogate"] >= 1.7
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 148 * 128 + 1, 3 * 148 * 128 + 130])
+def test_forward_at_tile_edges_and_alignments(n):
+    """Row counts at the edges of a tile, of one tile an SM and of one a group;
+    features and outputs 4 bytes off a 16-byte boundary take the scalar loads
+    and give the same bits.  Rows are independent, so the reference is the
+    BF16-rounded network on every 97th of them."""
+    import torch
+
+    _, gz = _zone()
+    rng = np.random.default_rng(5)
+    w = mlp.init_weights(3)
+    gz.ctx.surrogate_set_params(weights=w, norm=_identity_norm())
+    X = rng.normal(size=(n, 12)).astype(np.float32)
+    out = []
+    for off in (0, 1):
+        Xd = torch.empty(n * 12 + 4, dtype=torch.float32, device="cuda:0")
+        Yd = torch.full((n * 16 + 4,), 7.0, dtype=torch.float32, device="cuda:0")
+        Xd[off: off + n * 12] = torch.from_numpy(X.ravel()).to("cuda:0")
+        gz.ctx.surrogate_forward(Xd[off:].data_ptr(), n, Yd[off:].data_ptr())
+        y = Yd.cpu().numpy()
+        assert np.all(y[:off] == 7.0) and np.all(y[off + n * 16:] == 7.0)  # nothing beyond the table
+        out.append(y[off: off + n * 16].reshape(n, 16)[:, :11])
+    assert np.array_equal(out[0], out[1])
+    pick = np.unique(np.r_[np.arange(0, n, 97), n - 1])
+    wf = gz.ctx.surrogate_get_params()[0].astype(np.float64)
+    ref = mlp.forward(wf, X[pick].astype(np.float64), bf16_round=True)[0][:, :11]
+    assert np.abs(out[0][pick] - ref).max() / np.abs(ref).max() <= 1e-2
