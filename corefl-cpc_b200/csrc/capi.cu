@@ -14,7 +14,7 @@
 
 namespace cfk {
 cudaError_t launch_weno_air(const Zone &z, const Param &p, const int *var, cudaStream_t st, int *n_launch);
-int weno_air_default_tile(const Dims &d, int dir);
+int weno_air_default_tile(const Dims &d, int dir, int order);
 cudaError_t launch_weno_air_dir(const Zone &z, const Param &p, int dir, int var, cudaStream_t st);
 cudaError_t weno_air_init_attributes();
 cudaError_t launch_pv_air(const Zone &z, const Param &p, cudaStream_t st, int *n_launch);
@@ -118,7 +118,8 @@ struct Tiles {
   int var[3];
   explicit Tiles(const cfk_ctx *c) {
     for (int d = 0; d < 3; ++d)
-      var[d] = c->tile_auto && c->p.n_spec == 0 ? weno_air_default_tile(c->z.d, d) : c->tile_var[d];
+      var[d] = c->tile_auto && c->p.n_spec == 0 ? weno_air_default_tile(c->z.d, d, c->p.inviscid_scheme == 72 ? 7 : 5)
+                                           : c->tile_var[d];
   }
 };
 

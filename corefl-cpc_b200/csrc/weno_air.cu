@@ -358,17 +358,31 @@ cudaError_t launch_weno_air_dir(const Zone &z, const Param &p, int dir, int var,
   return w7 ? launch_dir<2, 7>(z, eps_ref, sn, th, var, st) : launch_dir<2, 5>(z, eps_ref, sn, th, var, st);
 }
 
-// The tile variant of a sweep that was neither tuned nor set.  On blocks of
-// more than one wave of CTAs (4 a SM) x 31x4, y 31x8 and z 15x16 are the
-// fastest (us per WENO7 sweep of 257 x 257 x 65, the three shapes: x 611, 586,
-// 565, y 592, 615, 621, z 741, 661, 670).  Below that a CTA's own latency
-// counts, and the y/z shape that takes its faces in one round instead of two
-// is faster (40 x 37 x 33: 18.6, 18.6, 14.5 us).
-int weno_air_default_tile(const Dims &d, int dir) {
-  if (dir == 0) return 2;
-  const long long ctas = (long long)((d.mx + 15) / 16) * ((d.ext(dir) + 14) / 15) * (dir == 1 ? d.mz : d.my);
-  if (ctas <= 4 * 148) return 2;
-  return dir == 1 ? 0 : 1;
+// The tile variant of a sweep that was neither tuned nor set: the shape whose
+// tiles, cut to the extent's multiples, compute the fewest faces, a staged
+// point counting a tenth of one.  us per sweep of the three shapes and the choice:
+// x (63x2, 15x8, 31x4), 161 nodes 250, 246, 254; 200 (WENO5) 462, 440, 424; 257
+// 611, 586, 565.  y/z (31x8, 15x16, 7x16), 65 nodes 741, 661, 670; 97 289, 272,
+// 272; 113 256, 268, 279; 257 2320, 2402, 2447 -- the smallest each time (161 x 113 x
+// 97 as a whole 793 -> 783, a 257^3 RK3 step 28.68 -> 28.43 ms against fixed shapes).  A
+// sweep of one wave of CTAs (4 a SM) is as long as one CTA: there y and z take the
+// shape whose faces are one round a thread instead of two (40 x 37 x 33: 18.6,
+// 18.6, 14.5).
+int weno_air_default_tile(const Dims &d, int dir, int order) {
+  if (dir > 0 && (long long)((d.mx + 15) / 16) * ((d.ext(dir) + 14) / 15) * (dir == 1 ? d.mz : d.my) <= 4 * 148)
+    return 2;
+  const int len[2][3] = {{63, 15, 31}, {31, 15, 0}};
+  const int halo = order == 7 ? 8 : 6, *l = len[dir > 0], m = d.ext(dir);
+  int best = -1;
+  long long least = 0;
+  for (int v = 0; v < 3 && l[v] > 0; ++v) {
+    const long long cost = (long long)((m + l[v] - 1) / l[v]) * (10 * (l[v] + 1) + l[v] + halo);
+    if (best < 0 || cost < least) {
+      best = v;
+      least = cost;
+    }
+  }
+  return best;
 }
 
 // Host launcher: x, y and (3-D) z sweeps in the reference's order; var[d]
