@@ -33,15 +33,18 @@ struct MixVals {
 };
 
 // Tile shapes of a sweep (nodes per column TN x columns C); VAR is chosen per
-// direction by the tile autotuner.  Every shape has 256 faces, one a thread,
-// and at 128 registers and 81 to 97 KB two CTAs fit an SM: FP64-bound.  With
-// all 14 fields unrolled a face took 226 registers, one CTA an SM, and its code
-// did not fit the instruction cache (WENO5 of 2048 x 512: 1786 -> 558 us;
-// WENO7 of 90 x 70 x 60: 1561 -> 485 us).
+// direction by the tile autotuner.  Every shape has 128 faces, one a thread,
+// and at 128 registers and 43 to 59 KB four CTAs fit an SM (three of y/z 7x16):
+// FP64-bound.  Tiles of 256 faces in two CTAs an SM recompute less halo but put
+// half as many independent barriers in flight and leave a longer last wave:
+// 2048 x 512 WENO5 557 -> 510 us, 90 x 70 x 60 WENO7 478 -> 413 us, a 97 x 49 x
+// 33 Wu step 1956 -> 1896 us, and bitwise the same.  With all 14 fields unrolled
+// a face took 226 registers, one CTA of 256 an SM, and its code did not fit the
+// instruction cache (2048 x 512: 1786 us, 90 x 70 x 60: 1561 us).
 template <int DIR, int VAR>
 struct MixShape {
-  static constexpr int TN = DIR == 0 ? (VAR == 0 ? 63 : VAR == 1 ? 127 : 31) : (VAR == 0 ? 15 : VAR == 1 ? 31 : 63);
-  static constexpr int C = DIR == 0 ? (VAR == 0 ? 4 : VAR == 1 ? 2 : 8) : (VAR == 0 ? 16 : VAR == 1 ? 8 : 4);
+  static constexpr int TN = DIR == 0 ? (VAR == 0 ? 31 : VAR == 1 ? 63 : 15) : (VAR == 0 ? 15 : VAR == 1 ? 7 : 31);
+  static constexpr int C = DIR == 0 ? (VAR == 0 ? 4 : VAR == 1 ? 2 : 8) : (VAR == 0 ? 8 : VAR == 1 ? 16 : 4);
 };
 
 template <int DIR, int ORD, int NS, int VAR = 0>
@@ -52,7 +55,7 @@ struct MixTile {
   static constexpr int C = MixShape<DIR, VAR>::C;
   static constexpr int NF = TN + 1;
   static constexpr int NPT = TN + 2 * R + 2;
-  static constexpr int NT = 256;
+  static constexpr int NT = 128;
   static constexpr int NQ = MixVals<NS>::N;
   static constexpr int NV = 5 + NS;
   __device__ static int spt(int q, int c, int t) {
@@ -138,7 +141,7 @@ struct PPArgs {
 // HYB: hybrid UD/WENO scheme, the face switches on the shock sensor.
 // VAR: tile shape (MixShape).
 template <int DIR, int ORD, int NS, bool HYB, int VAR>
-__global__ void __launch_bounds__(256, 2) weno_mix_flux_diff(Zone z, double eps_ref,
+__global__ void __launch_bounds__(128, 4) weno_mix_flux_diff(Zone z, double eps_ref,
                                                              const __grid_constant__ Thermo thermo,
                                                              const double *sensor, double threshold, PPArgs pp) {
   using T = MixTile<DIR, ORD, NS, VAR>;

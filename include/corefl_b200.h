@@ -231,7 +231,7 @@ int cfk_compute_shock_sensor(cfk_ctx *ctx, void *stream);
 /* ---- tile autotuner (no reference counterpart) ---- */
 /* The WENO flux kernels come in CFK_TILE_VARIANTS tile shapes per sweep
  * (nodes per column x columns per CTA: x 63x2, 15x8, 31x4; y/z 31x8, 15x16,
- * 7x16 for air and, for mixtures, x 63x4, 127x2, 31x8; y/z 15x16, 31x8, 63x4).
+ * 7x16 for air and, for mixtures, x 31x4, 63x2, 15x8; y/z 15x8, 7x16, 31x4).
  * Until they are tuned or set, air sweeps choose by the bound block's size and
  * mixtures take variants {0, 0, 0}; the viscous form is 2 below.
  * cfk_autotune_tiles times each variant of each sweep on the bound zone (reps
