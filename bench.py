@@ -39,15 +39,14 @@ N_NODES = 257
 
 # FP64 operations of one WENO7 characteristic face flux (air) with its share
 # of the staging and flux difference, counted by the hardware: 2 x DFMA + DADD
-# + DMUL per face from ncu's instruction counters on a 161^3 block
-# (profiles/weno_air_flux_diff_161_fp64_counts.md; the same in all three
-# sweeps).  It includes the FMA/multiply steps into which divisions and square
-# roots expand.  The hand count of the restated arithmetic (each +, -, *, /,
-# sqrt = 1; fma = 2) is 2980: face set-up 93; per characteristic field the left
-# eigenvector row 14, projection of 8 points 186, two WENO7-Z sides 361, times
-# 5 fields; back-projection 44; staging share 30, difference share 10.
-FLOPS_PER_FACE_WENO7_CH = 3214.9
-FLOPS_PER_FACE_WENO7_CH_HAND = 2980.0
+# + DMUL from ncu's instruction counters on a 161^3 block, per face that a
+# tile computes (profiles/weno_air_flux_diff_161_fp64_counts.md: 2289 to 2348
+# in the three sweeps, the least is taken; the faces of partial tiles beyond
+# the block are in the counters and not in the numerator).  It includes the
+# Newton steps of the reciprocals and square roots.  The hand count of the same
+# arithmetic (each +, -, *, reciprocal, sqrt = 1; fma = 2) is 2200.
+FLOPS_PER_FACE_WENO7_CH = 2289.0
+FLOPS_PER_FACE_WENO7_CH_HAND = 2200.0
 
 
 # The reference's own CUDA kernels (its sources built unmodified for sm_100a,
@@ -879,7 +878,7 @@ def main():
                     "kernel": "weno_air_flux_diff<dir,7> (x/y/z sweeps)",
                     "peak_source": "measured live: cfk_measure_fp64_peak FMA-chain kernel",
                     "avg_launch_ms": avg_launch_ms, "flops_per_launch": FLOPS_PER_FACE_WENO7_CH * faces_per_launch,
-                    "flops_source": "ncu DFMA/DADD/DMUL counters per face, 161^3 "
+                    "flops_source": "ncu DFMA/DADD/DMUL counters per computed face, 161^3 "
                                     "(profiles/weno_air_flux_diff_161_fp64_counts.md)",
                     "frac_hand_count": FLOPS_PER_FACE_WENO7_CH_HAND * faces_per_launch / (avg_launch_ms * 1e-3)
                     / 1e12 / peak}
