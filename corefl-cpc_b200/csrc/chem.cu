@@ -302,8 +302,8 @@ __global__ void __launch_bounds__(kGroupBlock, kGroupCtas)
   SM &sm = *reinterpret_cast<SM *>(group_raw);
   load_group_tables<NS>(sm.tb, mech, threadIdx.x, kGroupBlock);
   for (int e = threadIdx.x; e < SM::kNodes; e += kGroupBlock) {
+    sm.mem[e].c[NS] = 1.0;
     sm.mem[e].g[NS] = 0.0;
-    sm.mem[e].act[NS] = 1.0;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;

@@ -6,10 +6,12 @@
 // warps hide it:
 //  * the lanes share the reactions (rates), the species (thermodynamics) and
 //    the columns of the matrix;
-//  * a rate of progress is kf' times the product of a_k = c_k exp(g_k) over
-//    the reactants or the products, kf' = A T^b exp(-Ea/T - sum of the
-//    reactants' g_k): with one exponential a species, the equilibrium constant
-//    costs a reaction no exponential and no division;
+//  * a forward rate takes one exponential and a backward one a second, of the
+//    difference of the sides' g_k: only that difference is as small as the
+//    reaction's own energy.  One exponential a species instead (activities
+//    c_k exp(g_k), and exp(-sum of the reactants' g_k) in the rate constant)
+//    carries the rounding of sums that reach 160 into every rate, and leaves
+//    the range of a double where g_k depends on an element's reference state;
 //  * the matrix is in molar units (rows and columns scaled by the molar
 //    masses), in which its diagonal is mostly the largest entry of its column,
 //    and is solved by Gauss-Jordan elimination with threshold pivoting in
@@ -18,7 +20,9 @@
 // Lanes a node, measured on 2^20 H2/air reactors of 4-64 substeps each and on
 // 1021 of them (ms): one, with the matrix in its registers, 31.9 and 2.72 (255
 // registers, 8 warps an SM, 80 000 cycles a substep); nine, a row each, 52.6
-// and 0.73 (a node takes four times the instructions); three, 26.0 and 0.71.
+// and 0.73 (a node takes four times the instructions); three, 26.0 and 0.71
+// with an exponential a species, 27.2 and 0.73 with one a backward rate, which
+// halves the time scale's error (3.5e-15 and 1.4e-15 against 64-bit values).
 // One lane with the matrix in shared memory, before, took 49.7 and 4.54.
 // Results match the runtime-count path to rounding.
 #pragma once
@@ -69,10 +73,10 @@ struct GroupTables {
 // ones, hit different banks.
 template <int NS>
 struct GroupMem {
-  double c[NS], w[NS];
-  double g[NS + 1], act[NS + 1];      // entry NS: no molecule (g 0, activity 1)
+  double w[NS];
+  double c[NS + 1], g[NS + 1];        // entry NS: no molecule (c 1, g 0)
   double q1[kMaxReac], q2[kMaxReac];  // rates of progress
-  static constexpr int kUsed = 4 * NS + 2 + 2 * kMaxReac;
+  static constexpr int kUsed = 3 * NS + 2 + 2 * kMaxReac;
   double pad[((3 - kUsed) % 16 + 16) % 16];
 };
 
@@ -211,18 +215,8 @@ __device__ __forceinline__ void group_rate(const GroupTables<NS> &tb, const Grou
                                            double lnT, double iT, double temp_t, double itemp_t, double &q1,
                                            double &q2) {
   const int type = tb.type[r];
-  const uint2 mol = tb.mol[r];
-  double gf = 0, af = 1, ab = 1;
-#pragma unroll
-  for (int k = 0; k < kMaxMol; ++k) {
-    const int i = mol.x >> 8 * k & 255u, j = mol.y >> 8 * k & 255u;
-    gf += S.g[i];
-    af *= S.act[i];
-    ab *= S.act[j];
-  }
-  const double ex = fma(tb.b[r], lnT, -tb.Ea[r] * iT);
-  double kf = tb.A[r] * exp(type > 4 ? ex : ex - gf);  // with exp(-gf) in it, except for the fall-off types
-  if (type == 3) kf = fma(tb.A2[r], exp(fma(tb.b2[r], lnT, -tb.Ea2[r] * iT) - gf), kf);
+  double kf = tb.A[r] * exp(fma(tb.b[r], lnT, -tb.Ea[r] * iT));
+  if (type == 3) kf = fma(tb.A2[r], exp(fma(tb.b2[r], lnT, -tb.Ea2[r] * iT)), kf);
   if (type > 3) {
     double cc = 0;
 #pragma unroll
@@ -236,29 +230,38 @@ __device__ __forceinline__ void group_rate(const GroupTables<NS> &tb, const Grou
         kf = 0;
       } else {
         const double pr = kf_low * cc * (1.0 / kf_high);
-        double F;  // ln of the broadening factor
+        kf = kf_high * pr * rcp_nr(1.0 + pr);
         if (type > 5) {
           const double al = tb.troe_alpha[r];
           double f_cent = fma(1 - al, exp(-t * tb.troe_it3[r]), al * exp(-t * tb.troe_it1[r]));
           if (type == 7) f_cent += exp(-tb.troe_t2[r] * iT);
-          // natural logarithms and one exponential for the broadening factor and exp(-gf)
+          // natural logarithms and one exponential for the broadening factor
           constexpr double per_ln10 = 0.43429448190325182765;
           const double lnFc = log(f_cent), logFc = lnFc * per_ln10;
           const double x = fma(log(pr), per_ln10, fma(-0.67, logFc, -0.4));
           const double tempo = x * rcp_nr(fma(-0.14, x, fma(-1.27, logFc, 0.75)));
-          F = lnFc * rcp_nr(fma(tempo, tempo, 1.0));
-        } else {
-          F = 0;
+          kf *= exp(lnFc * rcp_nr(fma(tempo, tempo, 1.0)));
         }
-        kf = kf_high * pr * rcp_nr(1.0 + pr) * exp(F - gf);
       }
     }
   }
+  const uint2 mol = tb.mol[r];
+  double dg = 0, af = 1, ab = 1;  // dg: g of the products less that of the reactants
+#pragma unroll
+  for (int k = 0; k < kMaxMol; ++k) {
+    const int i = mol.x >> 8 * k & 255u, j = mol.y >> 8 * k & 255u;
+    dg += S.g[j] - S.g[i];
+    af *= S.c[i];
+    ab *= S.c[j];
+  }
   q1 = kf * af;
-  // kb = kf / Kc carries (p_atm / R_u T)^-order
-  q2 = type != 0 ? kf * ab : 0.0;
-  const int o = tb.order[r];
-  for (int k = 0; k < (o < 0 ? -o : o); ++k) q2 *= o < 0 ? temp_t : itemp_t;
+  // kb = kf / Kc, Kc = (p_atm / R_u T)^order exp(-dg)
+  q2 = 0;
+  if (type != 0) {
+    q2 = kf * exp(dg) * ab;
+    const int o = tb.order[r];
+    for (int k = 0; k < (o < 0 ? -o : o); ++k) q2 *= o < 0 ? temp_t : itemp_t;
+  }
 }
 
 // A row is swapped in as pivot only if its entry is more than this many times
@@ -336,12 +339,10 @@ __device__ __forceinline__ bool group_substep(const Zone &z, const GroupTables<N
 #pragma unroll
   for (int k = 0; k < SPL; ++k) {
     const int i = k * GL + me.j;
-    const double c = s.rY[k] * tb.imw3[i];
     const double g = gibbs_one(tb.low[i], tb.high[i], me.t_low[k], me.t_mid[k], me.t_high[k], t, lnT, iT);
     if (me.own) {
-      S.c[i] = c;
+      S.c[i] = s.rY[k] * tb.imw3[i];
       S.g[i] = g;
-      S.act[i] = c * exp(g);
     }
   }
   __syncwarp();

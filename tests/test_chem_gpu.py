@@ -165,3 +165,57 @@ def test_reaction_step_at_group_edges(n, long_side):
         assert np.array_equal(ns_o, ns_r)
         assert rel_err(out["cv"], oz["cv"]) <= 1e-12
         assert rel_err(out["sv"], oz["sv"], momentum=()) <= 1e-11  # the smallest species, against its own maximum
+
+
+def _reference_state(mech, d):
+    """The mechanism with the enthalpy of every H atom shifted by R d: another
+    reference state of the element, which no reaction's energy depends on."""
+    import dataclasses
+
+    n_h = np.asarray(mech.elem_comp)[:, list(mech.elements).index("H")]
+    low, high = np.array(mech.low), np.array(mech.high)
+    low[:, 5] += n_h * d
+    high[:, 5] += n_h * d
+    return dataclasses.replace(mech, low=low, high=high)
+
+
+def test_forward_rates_do_not_depend_on_the_elements_reference_state():
+    """One substep of an irreversible mechanism: the rates, and with them the
+    time scale, are those of A T^b exp(-Ea/T) and the concentrations alone, to
+    the last bit, whatever the species' g."""
+    import dataclasses
+
+    mech = mechanism.load("li2004")
+    mech = dataclasses.replace(mech, reac_type=np.zeros_like(mech.reac_type))
+    ts = []
+    for d in (0.0, 2e4, -2e4):
+        gz = GpuZone(cases.reactor_batch(_reference_state(mech, d), 256, seed=5))
+        gz.ctx.cv_from_bv()
+        gz.t["cv"][5:] += 1e-6 * gz.t["cv"][:1]  # all species present
+        gz.t["reaction_timeScale"].fill_(1.0)
+        gz.ctx.wu_reaction_step(1e-9, schedule=0)
+        ts.append(gz.get("reaction_timeScale"))
+    assert ts[0].min() > 0 and ts[0].max() < 1.0
+    assert np.array_equal(ts[0], ts[1]) and np.array_equal(ts[0], ts[2])
+
+
+@pytest.mark.parametrize("d", [4e5, -4e5])
+@pytest.mark.parametrize("schedule", [0, 1])
+def test_reaction_step_with_a_remote_reference_state(schedule, d):
+    """g of the hydrogen species beyond the range of exp (|d| / T > 709 a pair
+    of atoms) while most of them are absent: only differences of g enter.
+    Bar: g of some 900 carries about 5 roundings, four species a reaction, so
+    the rates of both sides differ by 4 x 5 x 900 x 2^-53 = 2e-12, of which a
+    step of 1e-7 s takes its share in 5 to 25 substeps."""
+    mech = _reference_state(mechanism.load("li2004"), d)
+    case = cases.reactor_batch(mech, 121, seed=8)
+    oz, gz = _pair(case)
+    oz["reaction_timeScale"][:] = 1e-7 / (0.5 + 5 + np.arange(121) % 20)
+    for _ in range(3):
+        gz.load_from(oz, keys=("cv", "bv", "sv", "reaction_timeScale"))
+        gz.ctx.wu_reaction_step(1e-7, schedule=schedule)
+        gz.ctx.sync()
+        oz.reaction_step(1e-7)
+        assert np.all(np.isfinite(gz.get("cv")))
+        assert rel_err(gz.get("cv"), oz["cv"]) <= 1e-10
+        assert rel_err(gz.get("bv")[[0, 4, 5]], oz["bv"][[0, 4, 5]], momentum=()) <= 1e-10
