@@ -52,7 +52,13 @@ struct Zone {
 // approximation (PTX rcp.approx.ftz.f64) and one third-order Householder step
 // y (1 + e + e^2), e = 1 - x y, whose remainder e^3 is below 2^-60; the result
 // is within 2 ulp.  Three FMAs, against a division sequence with its range
-// checks.  x = 0 and x = inf give NaN.
+// checks.  x = 0 and x = inf give NaN, where a division gives inf and 0, so it
+// stands only where x is neither for any state that has a finite answer:
+// densities, temperatures, Jacobians, sound speeds and sums of them; WENO
+// denominators (between eps^4 and the eighth power of a flux); the HLLC wave
+// speeds' differences (sl < 0 <= sm or sm < 0 <= sr in the star states); mixing sums
+// with positive terms; and rates behind their own thresholds.  Elsewhere a
+// division is written.
 __device__ __forceinline__ double rcp_nr(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

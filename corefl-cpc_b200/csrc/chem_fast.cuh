@@ -229,18 +229,18 @@ __device__ __forceinline__ void group_rate(const GroupTables<NS> &tb, const Grou
       if (kf_high < 1e-25 && kf_low < 1e-25) {
         kf = 0;
       } else {
-        const double pr = kf_low * cc * (1.0 / kf_high);
+        const double pr = kf_low * cc / kf_high;  // kf_high can be subnormal
         kf = kf_high * pr * rcp_nr(1.0 + pr);
         if (type > 5) {
           const double al = tb.troe_alpha[r];
           double f_cent = fma(1 - al, exp(-t * tb.troe_it3[r]), al * exp(-t * tb.troe_it1[r]));
           if (type == 7) f_cent += exp(-tb.troe_t2[r] * iT);
-          // natural logarithms and one exponential for the broadening factor
+          // ln F = ln Fc / (1 + (x / n)^2), with one reciprocal, of n^2 + x^2: n passes zero
           constexpr double per_ln10 = 0.43429448190325182765;
           const double lnFc = log(f_cent), logFc = lnFc * per_ln10;
           const double x = fma(log(pr), per_ln10, fma(-0.67, logFc, -0.4));
-          const double tempo = x * rcp_nr(fma(-0.14, x, fma(-1.27, logFc, 0.75)));
-          kf *= exp(lnFc * rcp_nr(fma(tempo, tempo, 1.0)));
+          const double n = fma(-0.14, x, fma(-1.27, logFc, 0.75)), nn = n * n;
+          kf *= exp(lnFc * nn * rcp_nr(fma(x, x, nn)));
         }
       }
     }
