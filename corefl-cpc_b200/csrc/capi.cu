@@ -523,17 +523,19 @@ int cfk_set_mechanism(cfk_ctx *c, const cfk_mechanism *m) {
   }
   std::stable_sort(kn.order_sp, kn.order_sp + ns, [&](int x, int y) { return uses[x] > uses[y]; });
   for (int i = 0; i < ns; ++i) pos[kn.order_sp[i]] = i;
-  kn.lists_ok = 1;
-  for (int r = 0; r < m->n_reac; ++r)
-    for (int l = 0; l < ns; ++l) {
-      const int f = m->stoi_f[r][l], b = m->stoi_b[r][l];
-      if (kn.n_f[r] + f > kMaxMol || kn.n_b[r] + b > kMaxMol) {
-        kn.lists_ok = 0;
-        continue;
-      }
-      for (int k = 0; k < f; ++k) kn.lf[r][kn.n_f[r]++] = (unsigned char)pos[l];
-      for (int k = 0; k < b; ++k) kn.lb[r][kn.n_b[r]++] = (unsigned char)pos[l];
+  for (int r = 0; r < m->n_reac; ++r) {
+    int f = 0, b = 0;
+    for (int q = 0; q < kn.n_inv[r]; ++q) {
+      kn.inv_pos[r][q] = (unsigned char)pos[kn.inv_sp[r][q]];
+      f += kn.inv_f[r][q];
+      b += kn.inv_b[r][q];
     }
+    kn.long_side[r] = f > kMaxMol || b > kMaxMol;
+    for (int q = 0; q < kn.n_inv[r] && !kn.long_side[r]; ++q) {
+      for (int k = 0; k < kn.inv_f[r][q]; ++k) kn.lf[r][kn.n_f[r]++] = kn.inv_pos[r][q];
+      for (int k = 0; k < kn.inv_b[r][q]; ++k) kn.lb[r][kn.n_b[r]++] = kn.inv_pos[r][q];
+    }
+  }
   // reactions of like type next to each other, so that the lanes of a warp
   // diverge in few rounds of the deal
   for (int r = 0; r < m->n_reac; ++r) kn.deal[r] = (unsigned char)r;

@@ -293,7 +293,7 @@ struct GroupSmem {
 // its groups), so nodes with uneven substep counts do not leave the rest of
 // the warp idle.  With a node list, the queue runs over list[0 ..
 // *list_count) instead of all nodes.  Otherwise group i takes node i.
-template <int NS, int GL, bool QUEUE>
+template <int NS, int GL, bool QUEUE, bool LONG>
 __global__ void __launch_bounds__(kGroupBlock, kGroupCtas)
     wu_reaction_ns_kernel(Zone z, Param p, const __grid_constant__ Mech mech, double dt, int *nsub_out, int *err,
                           unsigned int *counter, const unsigned int *list, const unsigned int *list_count) {
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kGroupBlock, kGroupCtas)
   GroupMem<NS> &S = sm.mem[slot];
   const Dims d = z.d;
   const unsigned int total = list ? *list_count : (unsigned int)d.mx * d.my * d.mz;
-  const int n_reac = mech.kn.n_reac, method = p.chem_advance_method;
+  const int method = p.chem_advance_method;
   GroupState<NS / GL> s = {};
   s.T = 1000.0; s.q[0] = 1.0; s.iJac = 1.0;  // a state that computes, for the groups without a node
 #pragma unroll
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kGroupBlock, kGroupCtas)
     // substeps 0..n_sub-1 use h, the last one h_last (skipped if ~0)
     const double hh = done < n_sub ? h : h_last;
     const bool run = have && (done < n_sub || abs(h_last) > 1e-12);
-    if (__any_sync(0xffffffffu, run)) ok &= group_substep<NS, GL>(z, sm.tb, S, me, n_reac, method, hh, run, s);
+    if (__any_sync(0xffffffffu, run)) ok &= group_substep<NS, GL, LONG>(z, mech.kn, sm.tb, S, me, method, hh, run, s);
     if (run) ++taken;
     if (have && ++done > n_sub) {
       if (!ok && me.j == 0) atomicOr(err, 1);
@@ -369,21 +369,32 @@ __global__ void __launch_bounds__(kGroupBlock, kGroupCtas)
   }
 }
 
-template <bool QUEUE>
-static cudaError_t launch_group_kernel(const Zone &z, const Param &p, const Mech &mech, double dt, int *nsub_out,
-                                       int *err, unsigned int *counter, const unsigned int *list,
-                                       const unsigned int *list_count, long long nodes, int n_sm, cudaStream_t st) {
+template <bool QUEUE, bool LONG>
+static cudaError_t launch_group_variant(const Zone &z, const Param &p, const Mech &mech, double dt, int *nsub_out,
+                                        int *err, unsigned int *counter, const unsigned int *list,
+                                        const unsigned int *list_count, long long nodes, int n_sm, cudaStream_t st) {
   constexpr int smem = (int)sizeof(GroupSmem<kMaxSpec, kGroupLanes>),
                 per_cta = GroupSmem<kMaxSpec, kGroupLanes>::kNodes;
-  cudaError_t e = cudaFuncSetAttribute(wu_reaction_ns_kernel<kMaxSpec, kGroupLanes, QUEUE>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  auto kernel = wu_reaction_ns_kernel<kMaxSpec, kGroupLanes, QUEUE, LONG>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   long long blocks = (nodes + per_cta - 1) / per_cta;
   if (QUEUE && blocks > (long long)n_sm * kGroupCtas) blocks = (long long)n_sm * kGroupCtas;
   if (blocks < 1) blocks = 1;
-  wu_reaction_ns_kernel<kMaxSpec, kGroupLanes, QUEUE><<<(unsigned)blocks, kGroupBlock, smem, st>>>(
-      z, p, mech, dt, nsub_out, err, counter, list, list_count);
+  kernel<<<(unsigned)blocks, kGroupBlock, smem, st>>>(z, p, mech, dt, nsub_out, err, counter, list, list_count);
   return cudaGetLastError();
+}
+
+template <bool QUEUE>
+static cudaError_t launch_group_kernel(const Zone &z, const Param &p, const Mech &mech, double dt, int *nsub_out,
+                                       int *err, unsigned int *counter, const unsigned int *list,
+                                       const unsigned int *list_count, long long nodes, int n_sm, cudaStream_t st) {
+  bool long_side = false;
+  for (int r = 0; r < mech.kn.n_reac; ++r) long_side |= mech.kn.long_side[r] != 0;
+  return long_side ? launch_group_variant<QUEUE, true>(z, p, mech, dt, nsub_out, err, counter, list, list_count,
+                                                       nodes, n_sm, st)
+                   : launch_group_variant<QUEUE, false>(z, p, mech, dt, nsub_out, err, counter, list, list_count,
+                                                        nodes, n_sm, st);
 }
 
 cudaError_t launch_finite_rate_chemistry(const Zone &z, const Mech *mc, cudaStream_t st) {
@@ -395,7 +406,7 @@ cudaError_t launch_wu_reaction(const Zone &z, const Param &p, const Mech *mc, co
                                int schedule, int *nsub_out, int *err, unsigned int *counter, int n_sm,
                                cudaStream_t st) {
   const long long total = (long long)z.d.mx * z.d.my * z.d.mz;
-  if (p.n_spec == kMaxSpec && mc_host.kn.lists_ok) {
+  if (p.n_spec == kMaxSpec) {
     if (schedule == 0)
       return launch_group_kernel<false>(z, p, mc_host, dt, nsub_out, err, nullptr, nullptr, nullptr, total, n_sm, st);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
@@ -422,7 +433,7 @@ cudaError_t launch_wu_reaction_list(const Zone &z, const Param &p, const Mech *m
                                     int *err, unsigned int *counter, int n_sm, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
   if (e != cudaSuccess) return e;
-  if (p.n_spec == kMaxSpec && mc_host.kn.lists_ok)
+  if (p.n_spec == kMaxSpec)
     return launch_group_kernel<true>(z, p, mc_host, dt, nullptr, err, counter, list, list_count, max_nodes, n_sm, st);
   long long blocks = (long long)n_sm * 8;
   const long long need = (max_nodes + 127) / 128;

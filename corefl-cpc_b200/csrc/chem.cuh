@@ -15,7 +15,7 @@
 namespace cfk {
 
 constexpr int kMaxReac = 24;
-constexpr int kMaxMol = 3;       // molecules on one side of a reaction (species lists of the lane-group kernels)
+constexpr int kMaxMol = 3;       // molecules on one side of a reaction (molecule lists of the lane-group kernels)
 constexpr int kMaxInvolved = 6;  // distinct species appearing in one reaction
 
 struct Kinetics {
@@ -34,13 +34,12 @@ struct Kinetics {
   signed char stf[kMaxReac][kMaxSpec], stb[kMaxReac][kMaxSpec];
   unsigned int inv_mask[kMaxReac], net_mask[kMaxReac];
   // the same again for the lane-group kernels (chem_fast.cuh), species by
-  // their position in `order_sp` (the most involved first) and all factors as
-  // doubles: the reactants and products of a reaction, one entry a molecule
-  // (lists_ok = 0 where a side has more than kMaxMol of them); the reactions
-  // in the order they are dealt to the lanes; and, position by position, the
-  // reactions that involve the species
-  int lists_ok;
-  unsigned char order_sp[kMaxSpec];
+  // their position in `order_sp` (the most involved first): the reactants and
+  // products of a reaction, one entry a molecule, or, where a side has more
+  // than kMaxMol of them (long_side), inv_pos beside inv_f and inv_b; the
+  // reactions in the order they are dealt to the lanes; and, position by
+  // position, the reactions that involve the species, factors as doubles
+  unsigned char order_sp[kMaxSpec], inv_pos[kMaxReac][kMaxInvolved], long_side[kMaxReac];
   unsigned char n_f[kMaxReac], n_b[kMaxReac], lf[kMaxReac][kMaxMol], lb[kMaxReac][kMaxMol];
   unsigned char deal[kMaxReac];
   int n_ent;

@@ -135,8 +135,7 @@ def test_ignition_of_the_reference_reactor_case():
 def test_reaction_step_at_group_edges(n, long_side):
     """Node counts around the nodes of a warp (10) and of a CTA (40), both
     schedules, uneven substep counts.  long_side: a reaction with four
-    molecules on a side, which the lane-group kernels' species lists do not
-    hold, takes the runtime-count kernels."""
+    molecules on a side, more than the lane-group kernels' molecule lists hold."""
     import dataclasses
 
     mech = mechanism.load("li2004")
