@@ -218,3 +218,67 @@ def test_reaction_step_with_a_remote_reference_state(schedule, d):
         assert np.all(np.isfinite(gz.get("cv")))
         assert rel_err(gz.get("cv"), oz["cv"]) <= 1e-10
         assert rel_err(gz.get("bv")[[0, 4, 5]], oz["bv"][[0, 4, 5]], momentum=()) <= 1e-10
+
+
+@pytest.mark.parametrize("mech_name", ["li2004", "premix_h2_ar"])
+@pytest.mark.parametrize("dt", [1e-6, 1e-5])
+def test_coarse_substeps_of_burning_states(mech_name, dt):
+    """One substep far beyond the time scale, where the matrix is far from the
+    identity and most nodes swap rows, from radical-rich states, both schedules.
+    Bar: a change of the matrix by a rounding (1e-16) changes the solution of
+    these systems by up to 4e-13 at 10 us, so rates that differ by rounding
+    (3e-15) give 1e-11."""
+    mech = mechanism.load(mech_name)
+    if mech_name == "li2004":
+        case = cases.reactor_batch(mech, 41, seed=3)
+    else:
+        X = np.zeros(mech.n_spec)
+        X[mech.index("H2")], X[mech.index("O2")], X[mech.index("AR")] = 0.2, 0.1, 0.7
+        case = cases.reactor(mech, np.linspace(1500.0, 1900.0, 41), 30000.0, X)
+    oz, gz = _pair(case)
+    for _ in range(40):
+        gz.ctx.wu_reaction_step(2e-7 if mech_name == "li2004" else 2e-6, schedule=1)
+    for k in ("cv", "bv", "sv"):
+        oz[k][:] = gz.get(k)
+    oz["reaction_timeScale"][:] = 2 * dt  # one substep
+    before = gz.get("sv").copy()
+    out = []
+    for schedule in (0, 1):
+        gz.load_from(oz, keys=("cv", "bv", "sv", "reaction_timeScale"))
+        gz.ctx.wu_reaction_step(dt, schedule=schedule)
+        gz.ctx.sync()
+        out.append([gz.get(k).copy() for k in ("cv", "sv", "reaction_timeScale")])
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+    ns = oz.reaction_step(dt, want_nsub=True)
+    assert np.all(ns == 1)
+    assert np.abs(out[0][1] - before).max() > 1e-5  # the step did something
+    assert rel_err(out[0][0], oz["cv"]) <= 1e-11
+    assert rel_err(out[0][1], oz["sv"], momentum=()) <= 1e-11
+
+
+@pytest.mark.parametrize("edge", ["t_low", "t_mid", "t_high", "cold"])
+def test_states_at_the_edges_of_the_thermo_ranges(edge):
+    """Temperatures on and one part in 1e6 around each end of the species' polynomial
+    ranges and at 250 to 350 K, with the radicals present or exactly zero."""
+    mech = mechanism.load("li2004")
+    if edge == "cold":
+        T = np.linspace(250.0, 350.0, 21)
+    else:
+        t = np.unique(np.asarray(getattr(mech, edge), dtype=float))
+        T = np.concatenate([t, t * (1 - 1e-6), t * (1 + 1e-6), t * 0.98, t * 1.02])
+    T = np.concatenate([T, T])
+    X = np.full((T.size, 9), 1e-4)
+    X[T.size // 2:] = 0.0
+    X[:, mech.index("H2")], X[:, mech.index("O2")], X[:, mech.index("N2")] = 0.3, 0.15, 0.55
+    case = cases.reactor(mech, T, 101325.0, X / X.sum(axis=1, keepdims=True))
+    oz, gz = _pair(case)
+    for step in range(2):
+        oz["reaction_timeScale"][:] = 1e-8 / 4.5
+        gz.load_from(oz, keys=("cv", "bv", "sv", "reaction_timeScale"))
+        gz.ctx.wu_reaction_step(1e-8, schedule=step)
+        gz.ctx.sync()
+        oz.reaction_step(1e-8)
+        assert rel_err(gz.get("cv"), oz["cv"]) <= 1e-12
+        assert rel_err(gz.get("bv")[[0, 4, 5]], oz["bv"][[0, 4, 5]], momentum=()) <= 1e-12
+        ts = oz["reaction_timeScale"]
+        assert np.all(np.abs(gz.get("reaction_timeScale") - ts) <= 1e-11 * np.abs(ts))
