@@ -469,7 +469,12 @@ int cfk_set_mechanism(cfk_ctx *c, const cfk_mechanism *m) {
     th.mw[l] = m->mw[l];
     th.imw[l] = 1.0 / m->mw[l];
     th.gas_const[l] = R_u / m->mw[l];
-    th.t_low[l] = m->t_low[l]; th.t_mid[l] = m->t_mid[l]; th.t_high[l] = m->t_high[l];
+    // the kernels pick the polynomial by t_mid alone, also for the ends of the range at which it is held
+    // outside: a t_mid beyond an end moves to it (past t_high, which still takes the lower polynomial)
+    th.t_low[l] = m->t_low[l]; th.t_high[l] = m->t_high[l];
+    th.t_mid[l] = !(m->t_mid[l] >= m->t_low[l]) ? m->t_low[l]
+                  : m->t_mid[l] > m->t_high[l]  ? std::nextafter(m->t_high[l], INFINITY)
+                                                : m->t_mid[l];
     for (int q = 0; q < 7; ++q) { th.low[l][q] = m->low[l][q]; th.high[l][q] = m->high[l][q]; }
     th.geometry[l] = m->geometry[l];
     th.LJ_potent_inv[l] = m->LJ_potent_inv[l];

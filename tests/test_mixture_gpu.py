@@ -128,3 +128,29 @@ def test_wu_splitting_reacting_tube_fixed_step():
     case.param["fixed_dt"] = 1
     case.param["dt"] = 1e-8
     _lockstep_wu(case, 3)
+
+
+@pytest.mark.parametrize("mid", ["above", "below"])
+def test_mid_temperature_outside_the_range(mid):
+    """A species table whose mid temperature lies beyond one end of its range
+    (a record with one range only): inside it the one polynomial, outside the
+    other at the end of the range, as the general formulas have it."""
+    import dataclasses
+
+    mech = mechanism.load("li2004")
+    T = cases.mix_wave(mech, 11).bv[5]
+    lo, hi, end = T.min(), T.max(), 0.5 * (T.min() + T.max())
+    assert hi - lo > 20
+    n = mech.n_spec
+    if mid == "above":
+        ranges = dict(t_low=np.full(n, lo - 100), t_mid=np.full(n, hi + 100), t_high=np.full(n, end))
+    else:
+        ranges = dict(t_low=np.full(n, end), t_mid=np.full(n, lo - 100), t_high=np.full(n, hi + 100))
+    case = cases.mix_wave(dataclasses.replace(mech, **ranges), 11)
+    oz = pyoracle.OracleZone(case)
+    oz.initialize()
+    gz = GpuZone(case)
+    gz.initialize()
+    for k in ("acoustic_speed", "gamma", "thermal_conductivity"):
+        assert rel_err(gz.get(k)[None], oz[k][None], momentum=()) <= 1e-13, k
+    assert rel_err(gz.get("cv"), oz["cv"]) <= 1e-14
