@@ -14,7 +14,7 @@
 
 namespace cfk {
 cudaError_t launch_weno_air(const Zone &z, const Param &p, const int *var, cudaStream_t st, int *n_launch);
-int weno_air_default_tile(const Dims &d, int dir, int order);
+int weno_air_default_tile(const Dims &d, int dir, int order, int n_sm);
 cudaError_t launch_weno_air_dir(const Zone &z, const Param &p, int dir, int var, cudaStream_t st);
 cudaError_t weno_air_init_attributes();
 cudaError_t launch_pv_air(const Zone &z, const Param &p, cudaStream_t st, int *n_launch);
@@ -28,7 +28,7 @@ cudaError_t launch_weno_mix_dir(const Zone &z, const Param &p, const Thermo &th,
 cudaError_t weno_mix_init_attributes();
 cudaError_t launch_viscous_mix(const Zone &z, const Param &p, const Thermo &th, cudaStream_t st, int *n_launch);
 cudaError_t viscous_mix_init_attributes();
-cudaError_t launch_viscous_air(const Zone &z, const Param &p, cudaStream_t st, int *n_launch, int var);
+cudaError_t launch_viscous_air(const Zone &z, const Param &p, cudaStream_t st, int *n_launch, int var, int n_sm);
 cudaError_t viscous_air_init_attributes();
 cudaError_t launch_update_rk(const Zone &z, const Param &p, const Thermo *th, double dt, const double *dt_dev,
                              int rk, int *err, cudaStream_t st, bool minus_cn = false, bool with_props = false);
@@ -118,17 +118,18 @@ struct Tiles {
   int var[3];
   explicit Tiles(const cfk_ctx *c) {
     for (int d = 0; d < 3; ++d)
-      var[d] = c->tile_auto && c->p.n_spec == 0 ? weno_air_default_tile(c->z.d, d, c->p.inviscid_scheme == 72 ? 7 : 5)
-                                           : c->tile_var[d];
+      var[d] = c->tile_auto && c->p.n_spec == 0
+                   ? weno_air_default_tile(c->z.d, d, c->p.inviscid_scheme == 72 ? 7 : 5, c->n_sm)
+                   : c->tile_var[d];
   }
 };
 
 // compute_viscous_flux dispatch (reference src/ViscousScheme.cu:7-73): the
 // 2nd-order face scheme or the 8th-order collocated one.
 cudaError_t launch_viscous(const Zone &z, const Param &p, const Thermo *th, const cfk_face *faces, int n_face,
-                           cudaStream_t st, int *n, int visc_var = 0) {
+                           cudaStream_t st, int *n, int visc_var, int n_sm) {
   if (p.viscous_order == 8 || p.viscous_order == 4) return launch_viscous8(z, p, th, faces, n_face, z.fvis8, st, n);
-  return th ? launch_viscous_mix(z, p, *th, st, n) : launch_viscous_air(z, p, st, n, visc_var);
+  return th ? launch_viscous_mix(z, p, *th, st, n) : launch_viscous_air(z, p, st, n, visc_var, n_sm);
 }
 
 int validate(const cfk_param *p, std::string &why) {
@@ -592,7 +593,8 @@ int cfk_compute_viscous_flux(cfk_ctx *c, void *stream) {
   if (c->hp.viscous_order == 0) return CFK_OK;
   if (int r = need_mech_for_mixture(c)) return r;
   int n = 0;
-  CFK_CHECK(c, launch_viscous(c->z, c->p, thermo_host(c), c->hp.faces, c->hp.n_face, S(stream), &n, c->visc_var),
+  CFK_CHECK(c, launch_viscous(c->z, c->p, thermo_host(c), c->hp.faces, c->hp.n_face, S(stream), &n, c->visc_var,
+                              c->n_sm),
             "viscous flux");
   c->launches += n;
   return CFK_OK;
@@ -676,9 +678,9 @@ int cfk_autotune_tiles(cfk_ctx *c, int reps, double *ms_out, int *choice_out, vo
     double best = 1e300;
     for (int var = 0; var < 3 && e == cudaSuccess; ++var) {
       int nl = 0;
-      e = launch_viscous_air(zt, pt, st, &nl, var);  // warm-up
+      e = launch_viscous_air(zt, pt, st, &nl, var, c->n_sm);  // warm-up
       if (e == cudaSuccess) e = cudaEventRecord(a, st);
-      for (int r = 0; r < reps && e == cudaSuccess; ++r) e = launch_viscous_air(zt, pt, st, &nl, var);
+      for (int r = 0; r < reps && e == cudaSuccess; ++r) e = launch_viscous_air(zt, pt, st, &nl, var, c->n_sm);
       if (e == cudaSuccess) e = cudaEventRecord(b, st);
       if (e == cudaSuccess) e = cudaEventSynchronize(b);
       float ms = 0;
@@ -920,7 +922,8 @@ static int rk3_step_async(cfk_ctx *c, cudaStream_t st) {
     CFK_CHECK(c, cudaMemsetAsync(z.dq, 0, N * p.n_var * sizeof(double), st), "dq memset");
     if (p.viscous_order > 0) {
       PhaseScope ps(c, CFK_PH_VISCOUS, st, &n);
-      CFK_CHECK(c, launch_viscous(z, p, thermo_host(c), c->hp.faces, c->hp.n_face, st, &n, c->visc_var), "viscous flux");
+      CFK_CHECK(c, launch_viscous(z, p, thermo_host(c), c->hp.faces, c->hp.n_face, st, &n, c->visc_var, c->n_sm),
+                "viscous flux");
     }
     if (c->have_mech && p.n_reac > 0) {
       // explicit chemical source of a reacting mixture (reference src/RK.cuh:147-149)
@@ -1025,7 +1028,8 @@ static int wu_splitting(cfk_ctx *c, int schedule, const WuReaction &rx, double *
   CFK_CHECK(c, cudaMemsetAsync(z.dq, 0, N * p.n_var * sizeof(double), st), "dq memset");
   if (p.viscous_order > 0) {
     PhaseScope ps(c, CFK_PH_VISCOUS, st, &n);
-    CFK_CHECK(c, launch_viscous(z, p, thermo_host(c), c->hp.faces, c->hp.n_face, st, &n, c->visc_var), "viscous flux");
+    CFK_CHECK(c, launch_viscous(z, p, thermo_host(c), c->hp.faces, c->hp.n_face, st, &n, c->visc_var, c->n_sm),
+              "viscous flux");
   }
   {
     PhaseScope ps(c, CFK_PH_INVISCID, st, &n);
@@ -1072,7 +1076,8 @@ static int wu_splitting(cfk_ctx *c, int schedule, const WuReaction &rx, double *
     CFK_CHECK(c, cudaMemsetAsync(z.dq, 0, N * p.n_var * sizeof(double), st), "dq memset");
     if (p.viscous_order > 0) {
       PhaseScope ps(c, CFK_PH_VISCOUS, st, &n);
-      CFK_CHECK(c, launch_viscous(z, p, thermo_host(c), c->hp.faces, c->hp.n_face, st, &n, c->visc_var), "viscous flux");
+      CFK_CHECK(c, launch_viscous(z, p, thermo_host(c), c->hp.faces, c->hp.n_face, st, &n, c->visc_var, c->n_sm),
+                "viscous flux");
     }
     {
       PhaseScope ps(c, CFK_PH_INVISCID, st, &n);

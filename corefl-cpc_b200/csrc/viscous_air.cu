@@ -511,10 +511,10 @@ int viscous_chunk(long long tiles, int mz, int n_sm) {
 // compute_viscous_flux for air (reference src/ViscousScheme.cu:7-40): one
 // launch for all directions; var 0 the staged kernel, 1 the ring kernel,
 // 2 the ring kernel with the L2 prefetch of the metric two planes ahead.
-cudaError_t launch_viscous_air(const Zone &z, const Param &p, cudaStream_t st, int *n_launch, int var) {
+cudaError_t launch_viscous_air(const Zone &z, const Param &p, cudaStream_t st, int *n_launch, int var, int n_sm) {
   const Dims &d = z.d;
   dim3 grid((d.mx + kFX - 1) / kFX, (d.my + kFY - 1) / kFY);
-  const int planes = viscous_chunk((long long)grid.x * grid.y, d.mz, 148);
+  const int planes = viscous_chunk((long long)grid.x * grid.y, d.mz, n_sm);
   grid.z = (d.mz + planes - 1) / planes;
   if (var == 1) viscous_air_ring<kCtas, false><<<grid, kFT, sizeof(RingSmem), st>>>(z, p.Pr, planes);
   else if (var == 2) viscous_air_ring<kCtas, true><<<grid, kFT, sizeof(RingSmem), st>>>(z, p.Pr, planes);

@@ -23,6 +23,7 @@
 // consecutive lanes, y/z tiles put consecutive i columns on them.
 #include "cfk_common.cuh"
 #include "weno.cuh"
+#include "weno_tiles.cuh"
 
 namespace cfk {
 
@@ -31,8 +32,8 @@ namespace {
 constexpr int kNQ = 13;  // staged values per point: Q0..4, G0..4, p, J/2, lambda
 
 // Tile shapes of a sweep: VAR selects one of the CFK_TILE_VARIANTS shapes
-// (nodes per column TN x columns C), chosen per direction by
-// weno_air_default_tile or the tile autotuner.  x tiles run along the lanes,
+// (nodes per column TN x columns C), chosen per direction by weno_air_tile
+// (weno_tiles.cuh) or the tile autotuner.  x tiles run along the lanes,
 // y/z tiles put C consecutive i columns on the lanes.  Tiles are small, one or
 // two faces a thread of a 128-thread CTA: four CTAs fit an SM and their
 // stage, face and difference phases overlap.  With the same 128 registers and
@@ -41,8 +42,7 @@ constexpr int kNQ = 13;  // staged values per point: Q0..4, G0..4, p, J/2, lambd
 // (128 x 3) to 1100 (192 x 2).
 template <int DIR, int VAR>
 struct TileShape {
-  static constexpr int TN = DIR == 0 ? (VAR == 0 ? 63 : VAR == 1 ? 15 : 31) : (VAR == 0 ? 31 : VAR == 1 ? 15 : 7);
-  static constexpr int C = DIR == 0 ? (VAR == 0 ? 2 : VAR == 1 ? 8 : 4) : (VAR == 0 ? 8 : VAR == 1 ? 16 : 16);
+  static constexpr int TN = kAirTileNodes[DIR > 0][VAR], C = kAirTileColumns[DIR > 0][VAR];
 };
 
 template <int DIR, int ORD, int VAR = 0>
@@ -358,31 +358,9 @@ cudaError_t launch_weno_air_dir(const Zone &z, const Param &p, int dir, int var,
   return w7 ? launch_dir<2, 7>(z, eps_ref, sn, th, var, st) : launch_dir<2, 5>(z, eps_ref, sn, th, var, st);
 }
 
-// The tile variant of a sweep that was neither tuned nor set: the shape whose
-// tiles, cut to the extent's multiples, compute the fewest faces, a staged
-// point counting a tenth of one.  us per sweep of the three shapes and the choice:
-// x (63x2, 15x8, 31x4), 161 nodes 250, 246, 254; 200 (WENO5) 462, 440, 424; 257
-// 611, 586, 565.  y/z (31x8, 15x16, 7x16), 65 nodes 741, 661, 670; 97 289, 272,
-// 272; 113 256, 268, 279; 257 2320, 2402, 2447 -- the smallest each time (161 x 113 x
-// 97 as a whole 793 -> 783, a 257^3 RK3 step 28.68 -> 28.43 ms against fixed shapes).  A
-// sweep of one wave of CTAs (4 a SM) is as long as one CTA: there y and z take the
-// shape whose faces are one round a thread instead of two (40 x 37 x 33: 18.6,
-// 18.6, 14.5).
-int weno_air_default_tile(const Dims &d, int dir, int order) {
-  if (dir > 0 && (long long)((d.mx + 15) / 16) * ((d.ext(dir) + 14) / 15) * (dir == 1 ? d.mz : d.my) <= 4 * 148)
-    return 2;
-  const int len[2][3] = {{63, 15, 31}, {31, 15, 0}};
-  const int halo = order == 7 ? 8 : 6, *l = len[dir > 0], m = d.ext(dir);
-  int best = -1;
-  long long least = 0;
-  for (int v = 0; v < 3 && l[v] > 0; ++v) {
-    const long long cost = (long long)((m + l[v] - 1) / l[v]) * (10 * (l[v] + 1) + l[v] + halo);
-    if (best < 0 || cost < least) {
-      best = v;
-      least = cost;
-    }
-  }
-  return best;
+// The tile variant of a sweep that was neither tuned nor set.
+int weno_air_default_tile(const Dims &d, int dir, int order, int n_sm) {
+  return weno_air_tile(d.ext(dir), dir == 0 ? d.my : d.mx, dir == 2 ? d.my : d.mz, dir, order, n_sm);
 }
 
 // Host launcher: x, y and (3-D) z sweeps in the reference's order; var[d]
