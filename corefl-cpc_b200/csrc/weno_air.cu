@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(128, 4) weno_air_flux_diff(Zone z, double eps_
                                                               double threshold) {
   using T = AirTile<DIR, ORD, VAR>;
   constexpr int R = T::R, TN = T::TN, C = T::C, NF = T::NF, NPT = T::NPT;
+  static_assert(NF * C % T::NT == 0, "every lane of a warp comes to the __syncwarp of air_face in every round");
   extern __shared__ double sm[];
   double *spts = sm;
   double *sflx = sm + kNQ * C * NPT;

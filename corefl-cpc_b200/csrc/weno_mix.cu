@@ -147,6 +147,7 @@ __global__ void __launch_bounds__(128, 4) weno_mix_flux_diff(Zone z, double eps_
   using T = MixTile<DIR, ORD, NS, VAR>;
   using V = MixVals<NS>;
   constexpr int R = T::R, NPF = T::NPF, TN = T::TN, C = T::C, NF = T::NF, NPT = T::NPT;
+  static_assert(NF * C % T::NT == 0, "every lane of a warp comes to the __syncwarps of the face loop in every round");
   const Thermo *th = &thermo;
   extern __shared__ double sm[];
   double *spts = sm;
