@@ -32,7 +32,8 @@ def _corner(case, n, ny, nz):
         return np.ascontiguousarray(a.reshape(a.shape[:-3] + (-1,)))
 
     return dataclasses.replace(case, mx=n, my=ny, mz=nz, metric=cut(case.metric), jac=cut(case.jac), bv=cut(case.bv),
-                               sv=np.zeros((0, cut(case.jac).size)), x=None, xyz=None)
+                               sv=cut(case.sv) if case.sv.shape[0] else np.zeros((0, cut(case.jac).size)), x=None,
+                               xyz=None)
 
 
 @pytest.mark.parametrize("labels", list(LABELS))
@@ -70,3 +71,81 @@ def test_properties_shell_covers_what_the_update_leaves(shape):
     gz.ctx.properties()
     for k in keys:
         assert np.allclose(out[k], gz.get(k), rtol=1e-14, atol=0), k
+
+
+THIN = [(5, 9, 8), (6, 9, 8), (9, 5, 8), (9, 6, 8), (9, 8, 5), (9, 8, 6), (5, 5, 5), (4, 5, 6), (6, 4, 5), (5, 6, 4)]
+
+
+@pytest.mark.parametrize("kind", ["isothermal", "adiabatic", "back_pressure", "symmetry_wall"])
+@pytest.mark.parametrize("gas", ["air", "mixture"])
+@pytest.mark.parametrize("shape", THIN)
+def test_walls_and_back_pressure_of_thin_blocks(kind, gas, shape):
+    """The conditions whose ghosts read inner nodes up to ngg away, on blocks
+    of ngg, ngg + 1 and ngg + 2 nodes (ngg = 4) along each axis."""
+    mech = mechanism.load("li2004")
+    if gas == "air":
+        case = cases.perturbed(cases.sine_wave(n=13, ny=11, nz=11, scheme=72, viscous=True, amp=0.02), seed=1, amp=0.05)
+    else:
+        case = cases.perturbed(cases.mix_wave(mech, 13, ny=11, nz=11, scheme=72), seed=1, amp=0.01)
+    case = _corner(case, *shape)
+    if kind == "back_pressure":
+        case.faces = LABELS["outflow"]
+        case = cases.with_back_pressure(case, 0.9 * float(case.bv[4].mean()))
+    else:
+        if kind == "symmetry_wall":
+            case.faces = [(0, -1, 3), (1, -1, 2), (0, 1, 2), (1, 1, 3), (2, -1, 2), (2, 1, 2)]
+        else:
+            case.faces = [(a, d, 2) for a in range(3) for d in (-1, 1)]
+        catalytic = gas == "mixture" and kind == "isothermal"
+        case = cases.with_walls(case, thermal_type=int(kind == "adiabatic"), faces=(), catalytic_type=int(catalytic),
+                                yk=case.sv[:, 0] if catalytic else None)
+    oz = pyoracle.OracleZone(case)
+    oz.call("orc_compute_cv_from_bv")
+    gz = GpuZone(case)
+    gz.load_from(oz, keys=("cv", "bv"))
+    oz.call("orc_apply_boundary_conditions")
+    gz.ctx.boundary_conditions()
+    tol = 1e-14 if gas == "air" else 1e-13  # the mixture's energy is a sum over nine species' polynomials
+    for k in ("bv", "cv") + (("sv",) if gas == "mixture" else ()):
+        assert rel_err(gz.get(k), oz[k][: gz.t[k].shape[0]], momentum=()) <= tol, k
+
+
+@pytest.mark.parametrize("labels", ["periodic", "outflow"])
+@pytest.mark.parametrize("shape", THIN)
+def test_mixture_boundary_conditions_of_thin_blocks(labels, shape):
+    case = _corner(cases.perturbed(cases.mix_wave(mechanism.load("li2004"), 13, ny=11, nz=11, scheme=72), seed=3,
+                                   amp=0.01), *shape)
+    case.faces = LABELS[labels]
+    oz = pyoracle.OracleZone(case)
+    oz.call("orc_compute_cv_from_bv")
+    gz = GpuZone(case)
+    gz.load_from(oz, keys=("cv", "bv"))
+    oz.call("orc_apply_boundary_conditions")
+    gz.ctx.boundary_conditions()
+    for k in ("bv", "cv", "sv"):
+        assert rel_err(gz.get(k), oz[k][: gz.t[k].shape[0]], momentum=()) <= 1e-13, k
+
+
+@pytest.mark.parametrize("gas", ["air", "mixture"])
+@pytest.mark.parametrize("shape", [(2, 2, 2), (3, 3, 3), (2, 3, 9), (9, 2, 3), (3, 9, 2), (9, 7, 5)])
+def test_properties_shell_of_the_thinnest_blocks(gas, shape):
+    """As above with two and three nodes an axis, where an axis has no or one
+    inner node, and for air."""
+    if gas == "air":
+        case = cases.perturbed(cases.sine_wave(n=13, ny=11, nz=11, scheme=52, viscous=True, amp=0.02), seed=1, amp=0.02)
+        keys = ("mul",)
+    else:
+        case = cases.perturbed(cases.mix_wave(mechanism.load("li2004"), 13, ny=11, nz=11, scheme=52, dt=1e-9), seed=2,
+                               amp=1e-3)
+        keys = ("mul", "gamma", "acoustic_speed", "thermal_conductivity", "rho_D")
+    case = _corner(case, *shape)
+    case.faces = LABELS["outflow"]
+    gz = GpuZone(case)
+    gz.initialize()
+    for k in keys:
+        gz.t[k].mul_(1 + 1e-6)  # what the step does not write again stays off
+    gz.ctx.rk3_step()
+    out = {k: gz.get(k).copy() for k in keys}
+    gz.ctx.properties()
+    for k in keys:
+        assert np.all(np.isfinite(out[k])) and np.allclose(out[k], gz.get(k), rtol=1e-14, atol=0), k
