@@ -828,7 +828,7 @@ def main():
     ctx.cv_from_bv()
     ctx.sync()
     # tile shapes of the WENO sweeps, timed on this block (outside the timed region)
-    tiles, tile_ms = ([0, 0, 0], None) if args.no_autotune else ctx.autotune_tiles(reps=3)
+    tiles, tile_ms = ("by the block's size", None) if args.no_autotune else ctx.autotune_tiles(reps=3)
     visc_var, visc_ms = ctx.viscous_variant()
 
     for _ in range(args.warmup):

@@ -292,9 +292,10 @@ int cfk_create(const cfk_param *param, cfk_ctx **out) {
     p.limit_ll[l] = param->limit_ll[l];
     p.limit_ul[l] = param->limit_ul[l];
   }
-  // starting tile shapes and viscous form (cfk_autotune_tiles may change
-  // them); until they are tuned or set, the air sweeps choose by the bound
-  // block's size instead (weno_air_default_tile)
+  // Until the shapes are tuned or set, the air WENO sweeps choose by the bound
+  // block's size (weno_air_default_tile) and the mixtures' take the first;
+  // {2, 1, 1} is what cfk_autotune_tiles reports for the primitive-variable air
+  // schemes, which have one shape.
   if (p.n_spec == 0) {
     c->tile_var[0] = 2;
     c->tile_var[1] = 1;
@@ -514,7 +515,6 @@ int cfk_set_mechanism(cfk_ctx *c, const cfk_mechanism *m) {
         kn.stf[r][l] = (signed char)m->stoi_f[r][l];
         kn.stb[r][l] = (signed char)m->stoi_b[r][l];
         kn.inv_mask[r] |= 1u << l;
-        if (m->stoi_f[r][l] != m->stoi_b[r][l]) kn.net_mask[r] |= 1u << l;
         ++n;
       }
     }
@@ -672,7 +672,7 @@ int cfk_autotune_tiles(cfk_ctx *c, int reps, double *ms_out, int *choice_out, vo
       c->launches += reps + 1;
     }
   }
-  // the two forms of the fused air viscous kernel (staged, ring)
+  // the three forms of the fused air viscous kernel (staged, ring, ring with the L2 prefetch)
   int visc_choice = c->visc_var;
   if (e == cudaSuccess && !th && c->p.viscous_order == 2) {
     double best = 1e300;

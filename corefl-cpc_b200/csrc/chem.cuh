@@ -28,11 +28,10 @@ struct Kinetics {
   int n_inv[kMaxReac];
   int inv_sp[kMaxReac][kMaxInvolved];
   int inv_f[kMaxReac][kMaxInvolved], inv_b[kMaxReac][kMaxInvolved];
-  // the same stoichiometry dense per species, with bit masks of the species
-  // involved (inv_mask) and of those with a non-zero net coefficient
-  // (net_mask), for loops whose species index is a compile-time constant
+  // the same stoichiometry dense per species, with a bit mask of the species
+  // involved
   signed char stf[kMaxReac][kMaxSpec], stb[kMaxReac][kMaxSpec];
-  unsigned int inv_mask[kMaxReac], net_mask[kMaxReac];
+  unsigned int inv_mask[kMaxReac];
   // the same again for the lane-group kernels (chem_fast.cuh), species by
   // their position in `order_sp` (the most involved first): the reactants and
   // products of a reaction, one entry a molecule, or, where a side has more

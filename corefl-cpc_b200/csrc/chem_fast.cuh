@@ -286,8 +286,8 @@ __device__ __forceinline__ void group_rate(const Kinetics &kn, const GroupTables
 // same in all lanes; y receives the lane's unknowns.  The owner of a column
 // picks its pivot and passes its multipliers on.  Rows are swapped, by the whole
 // warp, only if some group's pivot is off the diagonal.  Swapping only where the
-// pivot is four times the diagonal is 0.6 % faster on 2^20 reactors (10 % where
-// substeps are 50 time scales), but its error on burning H2/O2/Ar at substeps
+// pivot is four times the diagonal is 0.6 % faster on 2^20 reactors (11 % at
+// substeps of 0.1 us, 15 % at 1 us), but its error on burning H2/O2/Ar at substeps
 // of 10 us and more is up to twice that of an LU factorisation with partial
 // pivoting; with partial pivoting here it is below that one's.
 template <int NS, int GL>

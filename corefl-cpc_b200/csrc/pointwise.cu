@@ -220,11 +220,11 @@ __global__ void update_physical_properties_kernel(Zone z, Param p, const Thermo 
   i -= g;
   j -= g;
   const int k = planar ? 0 : (int)blockIdx.y - g;
-  // shell: only the nodes the boundary conditions, the inner-face and halo
-  // assignments and the 2-D k-ghost copy can write — the ghost layers and the
-  // outermost interior layer; the update computed the others' properties
-  const bool inner = i >= 1 && i <= d.mx - 2 && j >= 1 && j <= d.my - 2 &&
-                     (d.mz == 1 ? k == 0 : (k >= 1 && k <= d.mz - 2));
+  // shell (2-D blocks; 3-D ones: shell_properties_kernel): only the nodes the
+  // boundary conditions, the inner-face and halo assignments and the k-ghost
+  // copy can write — the ghost layers and the outermost interior layer; the
+  // update computed the others' properties
+  const bool inner = i >= 1 && i <= d.mx - 2 && j >= 1 && j <= d.my - 2 && k == 0;
   const int64_t id = d.idx(g, i, j, k);
   if (!(shell && inner)) properties_point<MIX>(z, p, th, id);
   if (!planar) return;
@@ -243,7 +243,7 @@ __global__ void update_physical_properties_kernel(Zone z, Param p, const Thermo 
   }
 }
 
-// The shell of a 3-D block (see above) by its own index: of each axis the
+// The shell of a 3-D block by its own index: of each axis the
 // ghost layers and the outermost node on either side, first whole k planes,
 // then the j rows and last the i ends of what is left.  Launched over the
 // padded block, a warp in an interior row would compute for its few shell
@@ -360,7 +360,7 @@ __global__ void reset_dt_kernel(unsigned long long *bits) { *bits = (unsigned lo
 // ---------------------------------------------------------------------------
 // Boundary faces (reference src/BoundCond.cu:2002-2171, 3033-3080), each
 // over the face widened by ngg ghosts tangentially (reference
-// src/Mesh.cpp:14-31).  One thread per face node.
+// src/Mesh.cpp:14-31).  Threads a face node: face_work.
 // ---------------------------------------------------------------------------
 struct FaceGeom {
   int face, direction;

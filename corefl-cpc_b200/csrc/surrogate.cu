@@ -811,10 +811,10 @@ __global__ void __launch_bounds__(128, 1) sg_train_kernel(const __grid_constant_
       s = (long long)(((unsigned long long)a.perm_a * (unsigned long long)(a.start + r) + (unsigned long long)a.perm_b) %
                       (unsigned long long)a.n);
       for (int c = 0; c < kSgIn; ++c) x[c] = (a.X[s * kSgIn + c] - a.nrm.in_mean[c]) * a.nrm.in_rstd[c];
-        for (int c = 0; c < kSgOut; ++c) {
-          const float g = a.G[s * kSgOut + c], sc = a.nrm.out_scale[c];
-          tgt[c] = ((sc > 0.f ? asinhf(g / sc) : g) - a.nrm.out_mean[c]) / a.nrm.out_std[c];
-        }
+      for (int c = 0; c < kSgOut; ++c) {
+        const float g = a.G[s * kSgOut + c], sc = a.nrm.out_scale[c];
+        tgt[c] = ((sc > 0.f ? asinhf(g / sc) : g) - a.nrm.out_mean[c]) / a.nrm.out_std[c];
+      }
     } else {
       for (int c = 0; c < kSgIn; ++c) x[c] = 0.f;
       for (int c = 0; c < kSgOut; ++c) tgt[c] = 0.f;
@@ -887,11 +887,8 @@ __global__ void __launch_bounds__(128, 1) sg_train_kernel(const __grid_constant_
       }
     }
   }
-  {
-    double l = loss_acc;
-    for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
-    if (lane == 0) atomicAdd(a.loss, l);
-  }
+  for (int off = 16; off > 0; off >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, off);
+  if (lane == 0) atomicAdd(a.loss, loss_acc);
   fence_before_sync();
   __syncthreads();
   if (warp == 0) {

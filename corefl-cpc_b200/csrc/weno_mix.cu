@@ -34,7 +34,8 @@ struct MixVals {
 
 // Tile shapes of a sweep (nodes per column TN x columns C); VAR is chosen per
 // direction by the tile autotuner.  Every shape has 128 faces, one a thread,
-// and at 128 registers and 43 to 59 KB four CTAs fit an SM (three of y/z 7x16):
+// and at 128 registers and 40 to 58 KB four CTAs fit an SM (three of WENO7's
+// y/z 7x16, which has 58 KB):
 // FP64-bound.  Tiles of 256 faces in two CTAs an SM recompute less halo but put
 // half as many independent barriers in flight and leave a longer last wave:
 // 2048 x 512 WENO5 557 -> 510 us, 90 x 70 x 60 WENO7 478 -> 413 us, a 97 x 49 x

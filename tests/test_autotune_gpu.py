@@ -98,7 +98,7 @@ def test_autotune_mixture_and_pv_noop():
     assert all(0 <= c < 3 for c in choice) and all(t > 0 for row in ms for t in row)
     pv = GpuZone(cases.sod(64, 7, scheme=4))
     choice, ms = pv.ctx.autotune_tiles(reps=2)
-    # a no-op keeps the context's starting shapes (air: x 31x8, y/z 31x16)
+    # a no-op: these schemes have one shape a sweep, reported as {2, 1, 1} for air
     assert choice == [2, 1, 1] and all(t == 0 for row in ms for t in row)
 
 
@@ -106,7 +106,7 @@ def test_autotune_mixture_and_pv_noop():
 def test_viscous_forms_identical_and_in_parity(name):
     """The staged and the two cp.async-ring forms (the second with the L2
     prefetch of the metric) of the fused air viscous kernel
-    agree to the last bits (blocks not a multiple of the 32 x 8 x 32 tile, 2-D
+    agree to the last bits (blocks not a multiple of the 32 x 4 tile or a chunk, 2-D
     and 3-D, walls widening the boundary ranges) and each matches the oracle's
     viscous flux at the single-call bar."""
     if name == "wave_3d":
