@@ -835,25 +835,41 @@ __global__ void inner_face_kernel(Zone z, Zone tz, Param p, const Thermo *th, cf
 }
 
 // eliminate_k_gradient (reference src/FieldOperation.cu:47-72)
-// One thread a copied node: grid.z runs over the 2 ngg ghost planes.
-__global__ void eliminate_k_gradient_kernel(Zone z, Param p) {
+// One thread a node of plane 0 and array (grid.y: the arrays of bv, sv and cv),
+// which it reads once and writes to the 2 ngg ghost planes.  HBM-bound on large
+// planes.  us of the forms one thread for all arrays of a node, one a copied node
+// (plane 0 does not stay in L2 between the copies) and this one: air 2048 x 512
+// WENO5 156, 215, 107; mixture 521, 566, 276; air 16 x 4000 15, 21, 10; 48 x 7
+// 6.4, 6.3, 3.4.
+__global__ void eliminate_k_gradient_kernel(Zone z, Param p, int64_t plane) {
   const Dims d = z.d;
   const int g = d.ngg;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x - g;
-  const int j = blockIdx.y - g, k = (int)blockIdx.z < g ? (int)blockIdx.z - g : (int)blockIdx.z - g + 1;
-  if (i >= d.mx + g) return;
-  const int64_t sz = d.plane(g), i0 = d.idx(g, i, j, 0), ik = d.idx(g, i, j, k);
-#pragma unroll
-  for (int l = 0; l < 6; ++l) z.bv[ik + l * sz] = z.bv[i0 + l * sz];
-  for (int l = 0; l < p.n_scalar; ++l) z.sv[ik + l * sz] = z.sv[i0 + l * sz];
-#pragma unroll 5
-  for (int l = 0; l < p.n_var; ++l) z.cv[ik + l * sz] = z.cv[i0 + l * sz];
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= plane) return;
+  int l = blockIdx.y;
+  double *a = z.bv;
+  if (l >= 6) {
+    l -= 6;
+    a = z.sv;
+    if (l >= p.n_scalar) {
+      l -= p.n_scalar;
+      a = z.cv;
+    }
+  }
+  a += d.idx(g, -g, -g, 0) + t + l * d.plane(g);
+  const double v = *a;
+  for (int k = 1; k <= g; ++k) {
+    a[k * plane] = v;
+    a[-k * plane] = v;
+  }
 }
 
 static void launch_eliminate_k(const Zone &z, const Param &p, cudaStream_t st) {
   const int g = z.d.ngg;
   if (g < 1) return;
-  eliminate_k_gradient_kernel<<<dim3((z.d.mx + 2 * g + 127) / 128, z.d.my + 2 * g, 2 * g), 128, 0, st>>>(z, p);
+  const int64_t plane = z.d.stride(g, 2);
+  eliminate_k_gradient_kernel<<<dim3((unsigned)((plane + 127) / 128), 6 + p.n_scalar + p.n_var), 128, 0, st>>>(z, p,
+                                                                                                                plane);
 }
 
 // ---------------------------------------------------------------------------

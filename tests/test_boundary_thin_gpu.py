@@ -149,3 +149,28 @@ def test_properties_shell_of_the_thinnest_blocks(gas, shape):
     gz.ctx.properties()
     for k in keys:
         assert np.all(np.isfinite(out[k])) and np.allclose(out[k], gz.get(k), rtol=1e-14, atol=0), k
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (7, 5), (128, 3), (121, 17), (3, 300)])
+@pytest.mark.parametrize("gas", ["air", "mixture"])
+def test_k_copy_of_2d_blocks(gas, shape):
+    """Every ghost plane of bv, sv and cv is a copy of plane 0, corners
+    included, and plane 0 is left as it is."""
+    import torch
+
+    case = cases.sod(12, 7, scheme=52) if gas == "air" else cases.mix_tube(mechanism.load("premix_h2_ar"), 12, 7)
+    g, (n, ny) = case.ngg, shape
+    P = (n + 2 * g) * (ny + 2 * g) * (1 + 2 * g)
+    case = dataclasses.replace(case, mx=n, my=ny, metric=np.ones((9, P)), jac=np.ones(P), bv=np.ones((6, P)),
+                               sv=np.ones((case.param["n_scalar"], P)), x=None, xyz=None)
+    gz = GpuZone(case)
+    gen = torch.Generator(device="cuda:0").manual_seed(1)
+    keys = ("bv", "cv") + (("sv",) if gas == "mixture" else ())
+    before = {}
+    for k in keys:
+        gz.t[k].copy_(torch.rand(gz.t[k].shape, generator=gen, device="cuda:0", dtype=torch.float64))
+        before[k] = gz.t[k].clone().view(gz.t[k].shape[0], 1 + 2 * g, ny + 2 * g, n + 2 * g)
+    gz.ctx.eliminate_k_gradient()
+    for k in keys:
+        a = gz.t[k].view(before[k].shape)
+        assert torch.equal(a, before[k][:, g: g + 1].expand_as(a)), k
